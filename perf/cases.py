@@ -232,3 +232,26 @@ def tolerance(case):
     # P and the output are rounded to the input type (2^-9 or 2^-12 relative to nearest, each);
     # sums, maxima and the LSE are fp32.
     return {"rel": 1e-2} if case["dtype"] == "bf16" else {"rel": 2e-3}
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, in 64 bits: one head at a time, so that the scores of
+    the largest call fit the card several times over."""
+    c = dict(case)
+    s = prepare(c, seed)
+    mask = (s["mask"] if "mask" in s else _mask(c, None)).cuda()
+    q, k, v = (s[n].cuda() for n in ("q", "k", "v"))
+    out = torch.empty(q.shape, dtype=torch.float64, device="cuda")
+    lse = torch.empty(q.shape[:3], dtype=torch.float64, device="cuda")
+    for b in range(c["B"]):
+        m = mask[b, 0].double()
+        for h in range(c["H"]):
+            kv = h // (c["H"] // c["Hk"])
+            x = torch.addmm(m, q[b, h].double(), k[b, kv].double().T, alpha=1.0 / math.sqrt(c["d"]))
+            lse[b, h] = torch.logsumexp(x, dim=-1)
+            # a row that sees no key gives 0
+            p = x.sub_(lse[b, h].clamp_min(-1e300).unsqueeze(-1)).exp_()
+            out[b, h] = p @ v[b, kv].double()
+    if c["entry"] == "lse":
+        return out, lse
+    return out.cpu() if c["entry"] == "host" else out
