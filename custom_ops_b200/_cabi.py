@@ -30,6 +30,7 @@ EXPORTS = [
     "fa_mask_fwd_sm100_static_scratch",
     "fa_mask_build_sm100",
     "fa_mask_fwd_sm100_rule",
+    "fa_mask_fwd_sm100_rule_workspace_bytes",
     "fa_mask_fwd_sm100_combine",
     "fa_mask_fwd_sm100_combine_packed",
     "fa_mask_fwd_sm100_combine_peers",
@@ -139,6 +140,8 @@ def load(path: str | None = None):
         ctypes.c_void_p, ctypes.c_int64, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_uint32,
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
         ctypes.c_int32, ctypes.c_void_p]
+    lib.fa_mask_fwd_sm100_rule_workspace_bytes.restype = ctypes.c_int
+    lib.fa_mask_fwd_sm100_rule_workspace_bytes.argtypes = [P(FaMaskFwdArgs), ctypes.c_int32, P(ctypes.c_size_t)]
     lib.fa_mask_fwd_sm100_rule.restype = ctypes.c_int
     lib.fa_mask_fwd_sm100_rule.argtypes = [P(FaMaskFwdArgs), ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
                                            ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
@@ -267,6 +270,13 @@ def device_status(device: int = 0, clear: bool = True) -> int:
 
 
 RULE_WORKSPACE_BYTES = 16
+
+
+def rule_workspace_bytes(args: FaMaskFwdArgs, window: int) -> int:
+    """Bytes of workspace with which ``forward_rule`` may split the keys over the GPU."""
+    n = ctypes.c_size_t()
+    check(load().fa_mask_fwd_sm100_rule_workspace_bytes(ctypes.byref(args), int(window), ctypes.byref(n)))
+    return n.value
 
 
 def forward_rule(args: FaMaskFwdArgs, causal: int, window: int, valid_lens: int, stream: int,

@@ -156,7 +156,6 @@ torch::Tensor mha_fwd_rule_mask(const torch::Tensor& q, const torch::Tensor& k, 
         lens = valid_lens->to(q.device(), torch::kInt32).contiguous();
     }
     auto out = torch::empty_like(q);
-    auto ws = torch::empty({FA_SM100_RULE_WORKSPACE_BYTES}, torch::TensorOptions().dtype(torch::kUInt8).device(q.device()));
     FaMaskFwdArgs a{};
     a.struct_size = sizeof(FaMaskFwdArgs);
     a.device = q.get_device();
@@ -171,10 +170,15 @@ torch::Tensor mha_fwd_rule_mask(const torch::Tensor& q, const torch::Tensor& k, 
     a.seqlen_k = static_cast<int32_t>(Sk);
     a.head_dim = static_cast<int32_t>(d);
     a.dtype = is_bf16 ? FA_SM100_BF16 : FA_SM100_FP16;
+    size_t ws_bytes = 0;
+    int rc = fa_mask_fwd_sm100_rule_workspace_bytes(&a, static_cast<int32_t>(window), &ws_bytes);
+    TORCH_CHECK(rc == FA_SM100_OK, "mha_fwd_rule_mask: ", fa_mask_fwd_sm100_strerror(rc));
+    auto ws = torch::empty({static_cast<int64_t>(ws_bytes)},
+                           torch::TensorOptions().dtype(torch::kUInt8).device(q.device()));
     auto stream = at::cuda::getCurrentCUDAStream(q.get_device());
-    const int rc = fa_mask_fwd_sm100_rule(&a, causal ? 1 : 0, static_cast<int32_t>(window),
-                                          lens.defined() ? lens.data_ptr<int32_t>() : nullptr, ws.data_ptr(),
-                                          FA_SM100_RULE_WORKSPACE_BYTES, static_cast<void*>(stream.stream()));
+    rc = fa_mask_fwd_sm100_rule(&a, causal ? 1 : 0, static_cast<int32_t>(window),
+                                lens.defined() ? lens.data_ptr<int32_t>() : nullptr, ws.data_ptr(), ws_bytes,
+                                static_cast<void*>(stream.stream()));
     TORCH_CHECK(rc == FA_SM100_OK, "mha_fwd_rule_mask: ", fa_mask_fwd_sm100_strerror(rc));
     return out;
 }

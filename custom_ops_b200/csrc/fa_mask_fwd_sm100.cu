@@ -150,6 +150,14 @@ struct KParams {
     // (the launcher zeroes it on the stream before the kernel).
     int rule_causal, rule_window;
     const int* valid_lens;
+    // PACK kernels, for few rows or few units.  The query heads of one KV group are consecutive rows
+    // of one "head" (q, out, lse and the partials have that layout as they are), so H = Hk here and
+    // Sq = group size * pack_sq; row r of it is query r % pack_sq, and every tile reads the same pack_sq
+    // mask rows.  A rule launch whose units are cut or split is one of these too, packed or not
+    // (pack_sq = Sq): what a cut under a rule needs stays out of the kernel for many units, which it
+    // made 3 % slower (a causal window over 2048 keys: 65.9 us against 63.8).
+    int pack_sq;
+    unsigned int mask_panel_bytes;      // bytes of one mask panel load (PACK: fewer than 128 rows)
 };
 
 template <bool BF16>
@@ -266,7 +274,7 @@ struct Ring {
     }
 };
 
-template <int D, bool BF16, bool LIST, bool RULE = false>
+template <int D, bool BF16, bool LIST, bool RULE, bool PACK>
 __global__ void __launch_bounds__(kThreads, 1)
 fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k,
@@ -356,7 +364,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         int count = 0;
         if constexpr (LIST) {
             const unsigned char* fl = p.block_flags +
-                (static_cast<long long>(b) * p.m_pairs + mpair) * p.kv_blocks;
+                (PACK ? b : static_cast<long long>(b) * p.m_pairs + mpair) * p.kv_blocks;
             const uint32_t lst = blk_list + (k & 1) * (kMaxListBlocks * 2);
             for (int base_j = 0; base_j < p.kv_blocks; base_j += 32) {
                 const int jj = base_j + lane;
@@ -386,16 +394,42 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
             if constexpr (RULE) {
                 // the key blocks in which any row of the unit (both slots walk the same blocks)
                 // sees a key: between the first row's lower limit and the last row's upper one
+                // (packed heads: a unit may hold rows of any query, so all of them count)
                 const int rows = p.head_pairs ? kBlockM : 2 * kBlockM;
-                const int r_last = min(m0 + rows, p.Sq) - 1;
+                const bool packed = PACK && p.pack_sq != p.Sq;
+                const int sq = PACK ? p.pack_sq : p.Sq;
+                const int r_first = packed ? 0 : m0;
+                const int r_last = packed ? sq - 1 : min(m0 + rows, sq) - 1;
                 const int limit = p.valid_lens != nullptr ? min(p.Sk, p.valid_lens[b]) : p.Sk;
-                const int hi = p.rule_causal ? min(limit - 1, r_last + p.Sk - p.Sq) : limit - 1;
-                const int lo = p.rule_window > 0 ? m0 + p.Sk - p.Sq - p.rule_window : -1;
+                const int hi = p.rule_causal ? min(limit - 1, r_last + p.Sk - sq) : limit - 1;
+                const int lo = p.rule_window > 0 ? r_first + p.Sk - sq - p.rule_window : -1;
                 begin = max(lo + 1, 0) / kBlockN;
                 end = hi >= 0 ? hi / kBlockN + 1 : 0;
                 if (end < begin) end = begin;
+                if constexpr (PACK) {
+                    const unsigned n_vis = static_cast<unsigned>(end - begin);
+                    if (part != kPartWhole) {
+                        // the pieces share the VISIBLE blocks; rounding down leaves the last piece, the
+                        // merging one, at least one block whenever there is any
+                        const unsigned pieces = static_cast<unsigned>(p.cut_units);
+                        const unsigned piece = blockIdx.x % pieces;
+                        const unsigned shift = n_vis >= 2 * pieces ? 1u : 0u;
+                        if (piece + 1 != pieces) end = begin + static_cast<int>((piece + 1) * n_vis / pieces - shift);
+                        if (piece != 0) begin += static_cast<int>(piece * n_vis / pieces - shift);
+                    } else if (dual) {
+                        // a CTA's share of the visible blocks, the larger half to slot 0; a slot 1 that is
+                        // left without a block does not exist, so it never stores over slot 0's partial
+                        const unsigned ng = static_cast<unsigned>(p.split_groups), g = static_cast<unsigned>(sgroup);
+                        const int gb = begin + static_cast<int>(g * n_vis / ng);
+                        const int ge = begin + static_cast<int>((g + 1) * n_vis / ng);
+                        const int half = (ge - gb + 1) / 2;
+                        begin = t == 0 ? gb : gb + half;
+                        end = t == 0 ? gb + half : ge;
+                        if (t == 1 && end == begin) end = begin - 1;
+                    }
+                }
             }
-            int n = on ? max(end - begin, 0) : -1;                 // -1: the slot does not exist
+            int n = on ? max(end - begin, (RULE && PACK) ? -1 : 0) : -1;     // -1: the slot does not exist
             if (LIST && on) n = count;                             // may be 0: nothing visible at all
             sts32(ui + 4 * (kUiSlot + 4 * t + kUiSplit), static_cast<uint32_t>(split));
             sts32(ui + 4 * (kUiSlot + 4 * t + kUiBegin), static_cast<uint32_t>(begin));
@@ -580,7 +614,8 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                     const uint32_t lst = blk_list + (k & 1) * (kMaxListBlocks * 2);
                     const int n_of[2] = {max(ui_get(ui, kUiSlot + kUiN), 0), max(ui_get(ui, kUiSlot + 4 + kUiN), 0)};
                     const int begin_of[2] = {ui_get(ui, kUiSlot + kUiBegin), ui_get(ui, kUiSlot + 4 + kUiBegin)};
-                    const int row0_of[2] = {ui_get(ui, kUiSlot + kUiRow0), ui_get(ui, kUiSlot + 4 + kUiRow0)};
+                    const int row0_of[2] = {PACK ? 0 : ui_get(ui, kUiSlot + kUiRow0),
+                                            PACK ? 0 : ui_get(ui, kUiSlot + 4 + kUiRow0)};
                     const int b = p.mask_bcast ? 0 : ui_get(ui, kUiB);
                     const int nmax = (RULE || p.test_stall_mask) ? 0 : max(n_of[0], n_of[1]);
                     for (int j = 0; ok && j < nmax; ++j) {
@@ -596,7 +631,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                                 if (!(ok = mbar_wait(bar_m_empty + 8 * i, ph[i] ^ 1u, abort_flag, p.status,
                                                      kStMaskEmpty)))
                                     continue;
-                                mbar_arrive_expect_tx(bar_m_full + 8 * i, kPanelBytes);
+                                mbar_arrive_expect_tx(bar_m_full + 8 * i, PACK ? p.mask_panel_bytes : kPanelBytes);
                                 tma_load_3d(sM + i * kPanelBytes, &tm_m, bar_m_full + 8 * i,
                                             blk * kBlockN + hf * 64, row0_of[t], b);
                                 ph[i] ^= 1u;
@@ -858,8 +893,8 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         // this thread's row inside a swizzled mask panel: 16-byte chunk c of row r
         // lives at r*128 + ((c ^ (r & 7)) << 4)
         const int mt = p.head_pairs ? 0 : t;             // whose mask panels this group reads
-        const uint32_t m_row_addr = sM + (2 * mt) * kPanelBytes + row_in_tile * 128;
-        const uint32_t m_xor = static_cast<uint32_t>(row_in_tile & 7) << 4;
+        uint32_t m_row_addr = sM + (2 * mt) * kPanelBytes + (PACK ? 0 : row_in_tile) * 128;
+        uint32_t m_xor = PACK ? 0u : static_cast<uint32_t>(row_in_tile & 7) << 4;
         const float2 scale2 = make_float2(p.scale, p.scale);
 
         int gstep = 0;               // key-block steps of this slot so far, over all units
@@ -888,13 +923,22 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 continue;
             }
             const int begin_t = ui_get(ui, kUiSlot + 4 * t + kUiBegin);
+            [[maybe_unused]] int query = 0;               // PACK: the query of this thread's row
+            if constexpr (PACK) {
+                if (!warm) query = (ui_get(ui, kUiSlot + 4 * t + kUiRow0) + row_in_tile) % p.pack_sq;
+                if constexpr (!RULE) {
+                    m_row_addr = sM + (2 * mt) * kPanelBytes + query * 128;
+                    m_xor = static_cast<uint32_t>(query & 7) << 4;
+                }
+            }
             // RULE: the keys this thread's row sees, (rule_lo, rule_hi]
             int rule_lo = -1, rule_hi = 0x3fffffff;
             if constexpr (RULE) {
                 if (!warm) {
                     const int bb = ui_get(ui, kUiB);
                     const int limit = p.valid_lens != nullptr ? min(p.Sk, p.valid_lens[bb]) : p.Sk;
-                    const int diag = ui_get(ui, kUiSlot + 4 * t + kUiRow0) + row_in_tile + p.Sk - p.Sq;
+                    const int diag = PACK ? query + p.Sk - p.pack_sq
+                                          : ui_get(ui, kUiSlot + 4 * t + kUiRow0) + row_in_tile + p.Sk - p.Sq;
                     rule_hi = p.rule_causal ? min(limit - 1, diag) : limit - 1;
                     rule_lo = p.rule_window > 0 ? diag - p.rule_window : -1;
                 }
@@ -1710,7 +1754,7 @@ struct DeviceInfo {
     unsigned int* status_ptr = nullptr;
     unsigned int* status_host = nullptr;     // pinned, mapped: the kernels' copy of a wait that gave up
     bool status_host_failed = false;
-    bool attr_set[12] = {false, false, false, false, false, false, false, false, false, false, false, false};
+    bool attr_set[24] = {};                  // per kernel instantiation, see launch_fwd
     bool queried = false;
 };
 static DeviceInfo g_dev[kMaxDevices];
@@ -1819,22 +1863,70 @@ static unsigned long long next_cut_tag() {
     return g_cut_tag.fetch_add(1) + 1;
 }
 
-static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan) {
+// The problem as the kernel sees it.  With few query rows and grouped heads, the rows of all heads
+// of a KV group are packed into one "head" (KParams.pack_sq): a decode step then reads every key
+// block once per group instead of once per pair of heads, and the heads left are few enough to split
+// the keys over the GPU (one row, 16 heads in groups of four, 8 x 4096 keys: 74 -> 27 us).  From 65
+// rows on a group of two fills two tiles either way, and the head pairs keep their finer tile skipping.
+constexpr int kPackMaxRows = 64;
+struct Shape {
+    int H, Hk, Sq;
+    int pack;          // query rows per head, 0: heads are not packed
+};
+static Shape kernel_shape(const FaMaskFwdArgs* a) {
+    const int group = a->heads / a->heads_k;
+    if (group > 1 && a->seqlen_q > 0 && a->seqlen_q <= kPackMaxRows && (a->disable & FA_SM100_NO_HEAD_PAIRS) == 0)
+        return {a->heads_k, a->heads_k, group * a->seqlen_q, a->seqlen_q};
+    return {a->heads, a->heads_k, a->seqlen_q, 0};
+}
+
+// A mask given by rules instead of a tensor (see KParams): what fa_mask_fwd_sm100_rule passes on.
+struct RuleSpec {
+    int causal, window;
+    const int* valid_lens;
+    unsigned int* counter;            // a word of device memory private to the launch, or NULL
+    bool may_split;                   // the caller brought the workspace that a split or a cut needs
+};
+// Key ranges up to this many blocks run as one pass of whole units under a rule, whose result does
+// not depend on the number of SMs; above it, half-empty launches are split (512 rows, 32 heads in
+// groups of four, 36 blocks: 75.9 -> 52.3 us).
+constexpr int kRuleWholeBlocks = 24;
+
+static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan, const RuleSpec* rule = nullptr) {
     int rc = validate(a);
     if (rc != FA_SM100_OK) return rc;
     DeviceInfo* dev = nullptr;
     query_device(a->device, &dev);
     std::memset(plan, 0, sizeof(*plan));
     const int d = a->head_dim;
-    int m_pairs = ceil_div(a->seqlen_q, 2 * kBlockM);
+    const Shape ks = kernel_shape(a);
+    int m_pairs = ceil_div(ks.Sq, 2 * kBlockM);
     const int nb = ceil_div(a->seqlen_k, kBlockN);
-    const long long base_ctas = static_cast<long long>(m_pairs) * a->heads * a->batch;
+    const long long base_ctas = static_cast<long long>(m_pairs) * ks.H * a->batch;
+    const bool one_tile = ks.Sq <= kBlockM;
+    // the most key blocks a unit can visit: a window bounds them
+    int nb_unit = nb;
+    if (rule != nullptr && rule->window > 0) {
+        const long long span = static_cast<long long>(rule->window) + (a->seqlen_q < 2 * kBlockM ? a->seqlen_q : 2 * kBlockM);
+        const long long most = (span + kBlockN - 1) / kBlockN + 1;
+        if (most < nb_unit) nb_unit = static_cast<int>(most);
+    }
+    const bool rule_split = rule != nullptr && rule->may_split && nb_unit > kRuleWholeBlocks;
     int splits = 1;
-    if (nb > 0 && base_ctas > 0) {
+    if (rule != nullptr) {
+        // One query tile: an even number of splits, two per CTA, for about one CTA per SM.
+        // (More than one tile: the units are cut in pieces instead, below.)
+        if (rule_split && one_tile && base_ctas > 0 && base_ctas * 5 < static_cast<long long>(dev->sm_count) * 4) {
+            long long groups = dev->sm_count / base_ctas;
+            if (groups > nb_unit / 8) groups = nb_unit / 8;
+            if (groups > FA_SM100_MAX_SPLITS / 2) groups = FA_SM100_MAX_SPLITS / 2;
+            if (groups >= 1) splits = static_cast<int>(2 * groups);
+        }
+    } else if (nb > 0 && base_ctas > 0) {
         if (a->num_splits > 0) {
             splits = a->num_splits;
         } else if (base_ctas * 5 < static_cast<long long>(dev->sm_count) * 4 &&
-                   nb >= (a->seqlen_q <= kBlockM ? 8 : 24)) {
+                   nb >= (one_tile ? 8 : 24)) {
             // Too few CTAs to fill the GPU: cut the key range so that about one CTA
             // lands on every SM, keeping at least four key blocks per CTA.  (With more than
             // one query tile a split costs a partial of 256 rows per CTA and a merge kernel
@@ -1852,8 +1944,7 @@ static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan) {
     }
     // One query tile and a split key range: a CTA takes two splits side by side (dual mode),
     // so aim for two splits per SM-filling CTA.
-    const bool one_tile = a->seqlen_q <= kBlockM;
-    if (one_tile && splits > 1 && a->num_splits == 0) {
+    if (rule == nullptr && one_tile && splits > 1 && a->num_splits == 0) {
         long long s2 = 2LL * splits;
         if (s2 > nb / 4) s2 = nb / 4;
         if (s2 > FA_SM100_MAX_SPLITS) s2 = FA_SM100_MAX_SPLITS;
@@ -1866,14 +1957,14 @@ static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan) {
     // Grouped-query heads with an even group size: a unit is two heads of one group over one
     // 128-row tile instead of one head over two tiles.  K/V traffic is the same, every mask
     // tile is fetched once for two heads, and key blocks are skipped per 128 rows.
-    const bool head_pairs = !dual && (a->heads / a->heads_k) % 2 == 0 &&
+    const bool head_pairs = !dual && (ks.H / ks.Hk) % 2 == 0 &&
                             (a->disable & FA_SM100_NO_HEAD_PAIRS) == 0;
-    if (head_pairs) m_pairs = ceil_div(a->seqlen_q, kBlockM);
-    const int heads_u = head_pairs ? a->heads / 2 : a->heads;
+    if (head_pairs) m_pairs = ceil_div(ks.Sq, kBlockM);
+    const int heads_u = head_pairs ? ks.H / 2 : ks.H;
     plan->num_splits = splits;
     plan->kv_blocks = nb;
     plan->blocks_per_split = bps;
-    plan->q_tiles_per_cta = (a->seqlen_q > kBlockM || head_pairs) ? 2 : 1;
+    plan->q_tiles_per_cta = (!one_tile || head_pairs) ? 2 : 1;
     plan->head_pairs = head_pairs ? 1 : 0;
     // Units of (split, 256-row query pair, head, batch), or (split, 128-row tile, pair of heads,
     // batch) with head_pairs.  Pair mode is persistent: one CTA per
@@ -1906,7 +1997,8 @@ static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan) {
     plan->tile_skip = (splits == 1 && nb >= 4 && nb <= kMaxListBlocks && a->seqlen_q > 0 &&
                        (a->disable & FA_SM100_NO_TILE_SKIP) == 0) ? 1 : 0;
     // (block flags, then the counter the attention kernel hands out its units from)
-    if (plan->tile_skip) ws += align256(static_cast<size_t>(a->batch) * m_pairs * nb) + 256;
+    // (packed heads: one region per batch element, every unit holds all of its mask rows)
+    if (plan->tile_skip) ws += align256(static_cast<size_t>(a->batch) * (ks.pack ? 1 : m_pairs) * nb) + 256;
     // More single-pass units than CTAs and a last round that is at most half full: its units
     // are done in P pieces by P CTAs each.  A piece costs an epilogue of its own and the first
     // piece about 1.5 key blocks' time per partial it merges (measured), so the piece count
@@ -1916,12 +2008,16 @@ static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan) {
     // and the grid grows to units x pieces.
     // There a piece has to pay for itself against the whole unit, not against an idle SM: not
     // below twelve key blocks.
+    // Under a rule, units differ in length and are handed out one by one once there are more of
+    // them than CTAs, which evens the last round out by itself: there only fewer units are cut.
     plan->unit_cut = 0;
-    if (!dual && splits == 1 && nb >= (units < dev->sm_count ? 12 : 6) && units > 0 &&
+    const bool may_cut = rule != nullptr ? rule_split && units < dev->sm_count
+                                         : nb >= (units < dev->sm_count ? 12 : 6);
+    if (!dual && splits == 1 && may_cut && units > 0 &&
         units % dev->sm_count != 0 && (a->disable & FA_SM100_NO_UNIT_CUT) == 0) {
         long long pieces = dev->sm_count / (units % dev->sm_count);
         long long best = 2;
-        while ((best + 1) * (best + 1) * 100 <= 65LL * nb) ++best;     // floor(sqrt(0.65 nb)), at least 2
+        while ((best + 1) * (best + 1) * 100 <= 65LL * nb_unit) ++best;     // floor(sqrt(0.65 nb)), at least 2
         if (pieces > best) pieces = best;
         if (pieces >= 2) {
             plan->unit_cut = static_cast<int32_t>(pieces);
@@ -1946,9 +2042,9 @@ static int get_encode() {
 }
 
 // (planes, rows, cols) 16-bit tensor with element pitches `row_pitch` and `plane_pitch`,
-// read in boxes of 128 rows x 64 columns with the 128-byte swizzle.
+// read in boxes of `box_rows` x 64 columns with the 128-byte swizzle.
 static int encode_map(CUtensorMap* tm, const void* ptr, int dtype, int planes, int rows, int cols,
-                      long long row_pitch, long long plane_pitch) {
+                      long long row_pitch, long long plane_pitch, int box_rows = kBlockM) {
     const cuuint64_t dims[3] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows),
                                 static_cast<cuuint64_t>(planes)};
     // A single plane still needs a legal (multiple of 16 bytes, non-zero) outer stride.
@@ -1956,7 +2052,7 @@ static int encode_map(CUtensorMap* tm, const void* ptr, int dtype, int planes, i
     if (plane_pitch <= 0) plane_pitch = static_cast<long long>(rows) * row_pitch;
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(row_pitch) * 2,
                                    static_cast<cuuint64_t>(plane_pitch) * 2};
-    const cuuint32_t box[3] = {64, 128, 1};
+    const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = g_encode(
         tm, dtype == FA_SM100_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
@@ -1974,6 +2070,7 @@ struct MapKey {
     const void* q; const void* k; const void* v; const void* mask;
     long long mask_rs, mask_bs;
     int dtype, B, H, Hk, Sq, Sk, d, device;
+    int mask_rows, mask_box;          // rows of a mask plane, rows of one panel load
 };
 struct MapEntry {
     MapKey key;
@@ -2003,8 +2100,8 @@ static int get_maps(const MapKey& key, CUtensorMap* tq, CUtensorMap* tk, CUtenso
     if ((rc = encode_map(tv, key.v, key.dtype, key.B * key.Hk, key.Sk, key.d, key.d,
                          static_cast<long long>(key.Sk) * key.d)) != FA_SM100_OK) return rc;
     // mask: (batch, Sq rows, Sk columns); reads beyond either extent return 0
-    if ((rc = encode_map(tm, key.mask, key.dtype, key.mask_bs == 0 ? 1 : key.B, key.Sq, key.Sk, key.mask_rs,
-                         key.mask_bs)) != FA_SM100_OK) return rc;
+    if ((rc = encode_map(tm, key.mask, key.dtype, key.mask_bs == 0 ? 1 : key.B, key.mask_rows, key.Sk, key.mask_rs,
+                         key.mask_bs, key.mask_box)) != FA_SM100_OK) return rc;
     MapEntry& e = g_map_cache[g_map_next];
     g_map_next = (g_map_next + 1) % kMapCache;
     e.key = key;
@@ -2013,11 +2110,12 @@ static int get_maps(const MapKey& key, CUtensorMap* tq, CUtensorMap* tk, CUtenso
     return FA_SM100_OK;
 }
 
-template <int D, bool BF16, bool LIST, bool RULE = false>
-static int launch_fwd(DeviceInfo* dev, int slot, const CUtensorMap& tq, const CUtensorMap& tk,
+template <int D, bool BF16, bool LIST, bool RULE, bool PACK>
+static int launch_fwd(DeviceInfo* dev, const CUtensorMap& tq, const CUtensorMap& tk,
                       const CUtensorMap& tv, const CUtensorMap& tm, const KParams& kp, dim3 grid,
                       cudaStream_t stream, bool chained) {
-    auto kern = fa_mask_fwd_kernel<D, BF16, LIST, RULE>;
+    auto kern = fa_mask_fwd_kernel<D, BF16, LIST, RULE, PACK>;
+    const int slot = (D == 128 ? 0 : 1) + (BF16 ? 0 : 2) + (PACK ? 4 : 0) + (RULE ? 16 : LIST ? 8 : 0);
     if (!dev->attr_set[slot]) {
         // The in-kernel register re-balancing is only sound for the register count it was
         // written for; refuse to launch a build that came out different.
@@ -2384,18 +2482,21 @@ static void flag_cache_read(int device, int slot, cudaStream_t stream) {
     else cudaGetLastError();
 }
 
-// A mask given by rules instead of a tensor (see KParams): what fa_mask_fwd_sm100_rule passes on.
-struct RuleSpec {
-    int causal, window;
-    const int* valid_lens;
-    unsigned int* counter;            // a word of device memory private to the launch, or NULL
-};
+template <int D, bool BF16, bool PACK>
+static int launch_variant(bool list, bool rule, DeviceInfo* dev, const CUtensorMap& tq, const CUtensorMap& tk,
+                          const CUtensorMap& tv, const CUtensorMap& tm, const KParams& kp, dim3 grid,
+                          cudaStream_t stream, bool chained) {
+    if (rule) return launch_fwd<D, BF16, false, true, PACK>(dev, tq, tk, tv, tm, kp, grid, stream, chained);
+    if (list) return launch_fwd<D, BF16, true, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream, chained);
+    return launch_fwd<D, BF16, false, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream, chained);
+}
 
 static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_bytes,
                    cudaStream_t stream, bool adaptive_skip = true, const RuleSpec* rule = nullptr) {
     FaMaskFwdPlan plan;
-    int rc = make_plan(a, &plan);
+    int rc = make_plan(a, &plan, rule);
     if (rc != FA_SM100_OK) return rc;
+    const Shape ks = kernel_shape(a);
     const long long rows = static_cast<long long>(a->batch) * a->heads * a->seqlen_q;
     if (rows == 0) return FA_SM100_OK;
     if (a->q == nullptr || a->out == nullptr) return FA_SM100_ERR_NULL;
@@ -2464,7 +2565,7 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     }
     int* hint_counter = nullptr;
     const int region_rows = plan.head_pairs ? kBlockM : 2 * kBlockM;
-    const int regions = ceil_div(a->seqlen_q, region_rows);
+    const int regions = ceil_div(a->seqlen_q, region_rows);       // (packed heads: one)
     const size_t flag_bytes = static_cast<size_t>(a->batch) * regions * plan.kv_blocks;
     // (the remembered flags describe the caller's own buffer: not for a re-pitched copy, whose
     // address changes with the workspace, and not for the entry point that keeps no state)
@@ -2513,14 +2614,18 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     kp.o_part = o_part;
     kp.lse_part = lse_part;
     kp.status = dev->status_ptr;
-    kp.B = a->batch; kp.H = a->heads; kp.Hk = a->heads_k; kp.Sq = a->seqlen_q; kp.Sk = a->seqlen_k;
+    kp.B = a->batch; kp.H = ks.H; kp.Hk = ks.Hk; kp.Sq = ks.Sq; kp.Sk = a->seqlen_k;
+    const bool pack_kernel = ks.pack || (rule != nullptr && (plan.dual_split || plan.unit_cut));
+    kp.pack_sq = ks.pack ? ks.pack : ks.Sq;
+    const int mask_box = ks.pack ? (ks.pack + 7) & ~7 : kBlockM;
+    kp.mask_panel_bytes = static_cast<unsigned int>(mask_box) * 128u;
     kp.num_splits = plan.num_splits;
     kp.kv_blocks = plan.kv_blocks;
     kp.head_pairs = plan.head_pairs;
-    kp.m_pairs = plan.head_pairs ? ceil_div(a->seqlen_q, kBlockM) : ceil_div(a->seqlen_q, 2 * kBlockM);
+    kp.m_pairs = plan.head_pairs ? ceil_div(ks.Sq, kBlockM) : ceil_div(ks.Sq, 2 * kBlockM);
     kp.dual = plan.dual_split;
     kp.split_groups = plan.dual_split ? ceil_div(plan.num_splits, 2) : plan.num_splits;
-    kp.total_units = kp.m_pairs * kp.split_groups * (plan.head_pairs ? a->heads / 2 : a->heads) * a->batch;
+    kp.total_units = kp.m_pairs * kp.split_groups * (plan.head_pairs ? ks.H / 2 : ks.H) * a->batch;
     if (plan.unit_cut) {
         uint8_t* slots = static_cast<uint8_t*>(workspace) + plan.workspace_bytes - cut_bytes(plan.grid_x, d);
         // the partials are written with 256-bit stores; a workspace that is only 16-byte
@@ -2540,8 +2645,8 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
         kp.rule_causal = rule->causal;
         kp.rule_window = rule->window;
         kp.valid_lens = rule->valid_lens;
-        if (rule->counter != nullptr) {
-            // (a compare-and-swap counter that tolerates any content was measured first: with 148
+        if (rule->counter != nullptr && kp.cut_units == 0 && !plan.dual_split && kp.total_units > plan.grid_x) {
+            // (only where a CTA takes more than its first unit; a compare-and-swap counter that tolerates any content was measured first: with 148
             // CTAs drawing in waves its retries are quadratic and cost 100 us per launch)
             if (cudaMemsetAsync(rule->counter, 0, sizeof(unsigned int), stream) != cudaSuccess) return cuda_failed(__LINE__);
             kp.unit_counter = rule->counter;
@@ -2561,33 +2666,27 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     std::memset(&key, 0, sizeof(key));             // padding bytes take part in the compare
     key.q = a->q; key.k = a->k; key.v = a->v; key.mask = mask_ptr;
     key.mask_rs = mask_rs; key.mask_bs = mask_bs;
-    key.dtype = a->dtype; key.B = a->batch; key.H = a->heads; key.Hk = a->heads_k;
-    key.Sq = a->seqlen_q; key.Sk = a->seqlen_k; key.d = d; key.device = a->device;
+    key.dtype = a->dtype; key.B = a->batch; key.H = ks.H; key.Hk = ks.Hk;
+    key.Sq = ks.Sq; key.Sk = a->seqlen_k; key.d = d; key.device = a->device;
+    key.mask_rows = a->seqlen_q; key.mask_box = mask_box;
     if ((rc = get_maps(key, &tq, &tk, &tv, &tm)) != FA_SM100_OK) return rc;
 
     const dim3 grid(plan.grid_x, plan.grid_y, plan.grid_z);
     const bool chained = plan.mask_repitched || run_classify;
     const bool bf16 = a->dtype == FA_SM100_BF16;
     const bool list = kp.block_flags != nullptr;
-    const int slot = (d == 128 ? 0 : 2) + (bf16 ? 0 : 1) + (list ? 4 : 0) + (rule != nullptr ? 8 : 0);
-    if (rule != nullptr) {
-        // (a rule launch is a single pass without a skip list: fa_mask_fwd_sm100_rule sees to that)
-        if (list || plan.num_splits != 1 || plan.unit_cut != 0 || plan.mask_repitched) return FA_SM100_ERR_SHAPE;
-        if (d == 128) rc = bf16 ? launch_fwd<128, true, false, true>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained)
-                                : launch_fwd<128, false, false, true>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained);
-        else rc = bf16 ? launch_fwd<64, true, false, true>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained)
-                       : launch_fwd<64, false, false, true>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained);
-    } else if (d == 128) {
-        if (list) rc = bf16 ? launch_fwd<128, true, true>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained)
-                            : launch_fwd<128, false, true>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained);
-        else rc = bf16 ? launch_fwd<128, true, false>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained)
-                       : launch_fwd<128, false, false>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained);
-    } else {
-        if (list) rc = bf16 ? launch_fwd<64, true, true>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained)
-                            : launch_fwd<64, false, true>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained);
-        else rc = bf16 ? launch_fwd<64, true, false>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained)
-                       : launch_fwd<64, false, false>(dev, slot, tq, tk, tv, tm, kp, grid, stream, chained);
-    }
+    // (a rule launch has no skip list and nothing to re-pitch: fa_mask_fwd_sm100_rule sees to that)
+    if (rule != nullptr && (list || plan.mask_repitched)) return FA_SM100_ERR_SHAPE;
+    auto launch = [&](auto head_dim, auto is_bf16) {
+        constexpr int kD = decltype(head_dim)::value;
+        constexpr bool kBf16 = decltype(is_bf16)::value;
+        return pack_kernel ? launch_variant<kD, kBf16, true>(list, rule != nullptr, dev, tq, tk, tv, tm, kp, grid, stream, chained)
+                           : launch_variant<kD, kBf16, false>(list, rule != nullptr, dev, tq, tk, tv, tm, kp, grid, stream, chained);
+    };
+    if (d == 128) rc = bf16 ? launch(std::integral_constant<int, 128>{}, std::true_type{})
+                            : launch(std::integral_constant<int, 128>{}, std::false_type{});
+    else rc = bf16 ? launch(std::integral_constant<int, 64>{}, std::true_type{})
+                   : launch(std::integral_constant<int, 64>{}, std::false_type{});
     if (rc != FA_SM100_OK) return rc;
     if (flag_slot >= 0) flag_cache_read(a->device, flag_slot, stream);
     if (plan.num_splits > 1)
@@ -2633,6 +2732,23 @@ static int forward_static_scratch(const FaMaskFwdArgs* a, cudaStream_t stream) {
     }
     // (no adaptive pre-pass gating here: that would allocate a pinned host word)
     return forward(a, scratch, FA_SM100_STATIC_SCRATCH_BYTES, stream, /*adaptive_skip=*/false);
+}
+
+// A rule launch is the launch for a mask tensor without a pre-pass; the mask fields describe a
+// one-plane placeholder that no kernel reads.
+constexpr size_t kRuleCounterBytes = 256;
+static FaMaskFwdArgs rule_args(const FaMaskFwdArgs* args) {
+    FaMaskFwdArgs a = *args;
+    a.mask = a.q;
+    a.mask_seqlen_q = a.seqlen_q;
+    a.mask_seqlen_k = a.seqlen_k;
+    a.mask_row_stride = (static_cast<int64_t>(a.seqlen_k) + 7) & ~static_cast<int64_t>(7);
+    a.mask_batch_stride = 0;
+    a.num_splits = 1;
+    a.out_fp32 = 0;
+    a.mask_version = 0;
+    a.disable |= FA_SM100_NO_TILE_SKIP;
+    return a;
 }
 
 }  // namespace fa_sm100
@@ -2785,28 +2901,35 @@ int fa_mask_build_sm100(void* mask, int32_t batch, int32_t seqlen_q, int32_t seq
     return FA_SM100_OK;
 }
 
-int fa_mask_fwd_sm100_rule(const FaMaskFwdArgs* args, int32_t causal, int32_t window, const int32_t* valid_lens,
-                           void* workspace, size_t workspace_bytes, void* stream) {
-    if (args == nullptr) return FA_SM100_ERR_NULL;
+int fa_mask_fwd_sm100_rule_workspace_bytes(const FaMaskFwdArgs* args, int32_t window, size_t* bytes) {
+    if (args == nullptr || bytes == nullptr) return FA_SM100_ERR_NULL;
     if (args->struct_size != sizeof(FaMaskFwdArgs)) return FA_SM100_ERR_ABI;
     if (window < 0) return FA_SM100_ERR_SHAPE;
+    FaMaskFwdPlan plan;
+    const FaMaskFwdArgs a = fa_sm100::rule_args(args);
+    const fa_sm100::RuleSpec rule{0, window, nullptr, nullptr, true};
+    const int rc = fa_sm100::make_plan(&a, &plan, &rule);
+    if (rc != FA_SM100_OK) return rc;
+    *bytes = plan.workspace_bytes > 0 ? fa_sm100::kRuleCounterBytes + static_cast<size_t>(plan.workspace_bytes)
+                                      : FA_SM100_RULE_WORKSPACE_BYTES;
+    return FA_SM100_OK;
+}
+
+int fa_mask_fwd_sm100_rule(const FaMaskFwdArgs* args, int32_t causal, int32_t window, const int32_t* valid_lens,
+                           void* workspace, size_t workspace_bytes, void* stream) {
+    size_t full = 0;
+    const int rc = fa_mask_fwd_sm100_rule_workspace_bytes(args, window, &full);
+    if (rc != FA_SM100_OK) return rc;
     if (workspace != nullptr && (workspace_bytes < FA_SM100_RULE_WORKSPACE_BYTES ||
                                  (reinterpret_cast<uintptr_t>(workspace) & 15u) != 0))
         return FA_SM100_ERR_WORKSPACE;
-    // The same launch as for a mask tensor, as one pass over the keys with whole units and no
-    // pre-pass; the mask fields describe a one-plane placeholder that no kernel reads.
-    FaMaskFwdArgs a = *args;
-    a.mask = a.q;
-    a.mask_seqlen_q = a.seqlen_q;
-    a.mask_seqlen_k = a.seqlen_k;
-    a.mask_row_stride = (static_cast<int64_t>(a.seqlen_k) + 7) & ~static_cast<int64_t>(7);
-    a.mask_batch_stride = 0;
-    a.num_splits = 1;
-    a.out_fp32 = 0;
-    a.mask_version = 0;
-    a.disable |= FA_SM100_NO_TILE_SKIP | FA_SM100_NO_UNIT_CUT;
-    fa_sm100::RuleSpec rule{causal != 0 ? 1 : 0, window, valid_lens, static_cast<unsigned int*>(workspace)};
-    return fa_sm100::forward(&a, nullptr, 0, static_cast<cudaStream_t>(stream), true, &rule);
+    // [counter][partials of a split or the slots of a cut]; with less, one pass of whole units
+    const bool may_split = workspace != nullptr && full > fa_sm100::kRuleCounterBytes && workspace_bytes >= full;
+    const FaMaskFwdArgs a = fa_sm100::rule_args(args);
+    const fa_sm100::RuleSpec rule{causal != 0 ? 1 : 0, window, valid_lens, static_cast<unsigned int*>(workspace), may_split};
+    return fa_sm100::forward(&a, may_split ? static_cast<uint8_t*>(workspace) + fa_sm100::kRuleCounterBytes : nullptr,
+                             may_split ? workspace_bytes - fa_sm100::kRuleCounterBytes : 0,
+                             static_cast<cudaStream_t>(stream), true, &rule);
 }
 
 int fa_mask_fwd_sm100_static_scratch(const FaMaskFwdArgs* args, void* stream) {

@@ -57,8 +57,9 @@ enum {
     FA_SM100_NO_TILE_SKIP = 1,  /* visit every key block even where the mask hides it entirely */
     FA_SM100_NO_UNIT_CUT = 2,   /* every (query pair, head, batch) unit is finished by one CTA, so the
                                  * result does not depend on the number of SMs */
-    FA_SM100_NO_HEAD_PAIRS = 4, /* grouped-query heads are not paired: a unit is one head over a 256-row
-                                 * query pair, as for ungrouped heads */
+    FA_SM100_NO_HEAD_PAIRS = 4, /* grouped-query heads are neither paired nor, with few query rows, packed
+                                 * into shared query tiles: a unit is one head over a 256-row query pair,
+                                 * as for ungrouped heads */
     FA_SM100_TEST_STALL_MASK = 0x100  /* tests only: the kernel's mask loads are withheld and its waits
                                  * get a short limit (FA_SM100_TEST_WAIT_KCYCLES in the environment,
                                  * units of 1024 SM cycles, default 2000), so that a wait runs out,
@@ -204,15 +205,20 @@ int fa_mask_fwd_sm100_static_scratch(const FaMaskFwdArgs* args, void* stream);
  * exists in memory at all:  key j is visible to query row i when  lo < j <= hi,
  *   hi = min(limit - 1, causal ? i + Sk - Sq : +inf),   lo = window > 0 ? i + Sk - Sq - window : -1,
  *   limit = min(Sk, valid_lens[batch])  (Sk when valid_lens is NULL; a device array of `batch` ints).
- * Bit-identical to fa_mask_fwd_sm100 on the mask that fa_mask_build_sm100 writes for the same rules.
- * The mask fields of `args` are ignored (mask may be NULL); `lse` is honoured; one pass over the
- * keys whatever num_splits says.  `workspace`: FA_SM100_RULE_WORKSPACE_BYTES of device memory, 16-byte
- * aligned, that no other call uses until this one has finished - the counter the CTAs take their
- * units from (units differ in length under a rule; the call zeroes it on the stream with a
- * cudaMemsetAsync ahead of the kernel); NULL: every CTA takes a fixed
- * share of the units instead (slower where the lengths differ much).  The reference has no such
- * operator. */
+ * One pass over the keys is bit-identical to fa_mask_fwd_sm100 (num_splits = 1, NO_UNIT_CUT) on the
+ * mask that fa_mask_build_sm100 writes for the same rules.  The mask fields of `args` and num_splits
+ * are ignored (mask may be NULL); `lse` is honoured.  `workspace`: device memory, 16-byte aligned,
+ * that no other call uses until this one has finished; its content does not matter.
+ *   fa_mask_fwd_sm100_rule_workspace_bytes(): the call may split long key ranges over the GPU where
+ *       too few units would leave SMs idle (fp32 partials, merged; the rounding of the merge is then
+ *       the only difference);
+ *   FA_SM100_RULE_WORKSPACE_BYTES: one pass; the counter the CTAs take their units from (units differ
+ *       in length under a rule; the call zeroes it on the stream with a cudaMemsetAsync ahead of the
+ *       kernel);
+ *   NULL: one pass, every CTA takes a fixed share of the units (slower where the lengths differ much).
+ * The reference has no such operator. */
 #define FA_SM100_RULE_WORKSPACE_BYTES 16
+int fa_mask_fwd_sm100_rule_workspace_bytes(const FaMaskFwdArgs* args, int32_t window, size_t* bytes);
 int fa_mask_fwd_sm100_rule(const FaMaskFwdArgs* args, int32_t causal, int32_t window, const int32_t* valid_lens,
                            void* workspace, size_t workspace_bytes, void* stream);
 

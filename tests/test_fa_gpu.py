@@ -815,3 +815,68 @@ def test_rule_attention_equals_the_operator_on_the_rule_mask(dtype, case):
         assert torch.equal(out2, want)
     assert _cabi.device_status(0, clear=True) == 0
 
+
+
+# ---------------------------------------------------------------- few query rows, grouped heads
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case", [
+    # b, h, hk, sq, sk, d, mask, forced splits
+    (2, 8, 2, 1, 700, 128, "drop10", 1),            # one pass, one slot of the CTA
+    (3, 8, 1, 7, 515, 64, "random", 1),             # 56 packed rows, ragged keys (mask is re-pitched)
+    (2, 4, 2, 64, 1024, 128, "block", 1),           # 128 packed rows: exactly one tile; skip list
+    (2, 6, 2, 63, 1411, 64, "causal", 1),           # 189 packed rows: two tiles, the second one ragged
+    (1, 16, 2, 33, 900, 128, "drop_bias", 1),       # 264 packed rows: a second unit of eight rows
+    (1, 8, 2, 1, 4096, 128, "drop10", 5),           # split keys, two splits per CTA, an odd one left over
+    (2, 8, 1, 40, 2053, 64, "random", 3),           # 320 packed rows, split keys
+])
+def test_packed_heads_equal_separate_heads(dtype, case):
+    """With at most 64 query rows the rows of all heads of a KV group share query tiles.  A row's
+    arithmetic does not depend on which rows it shares a tile with, so the result is bit-identical
+    to the run with one head per unit under the same splits."""
+    b, h, hk, sq, sk, d, kind, splits = case
+    q, k, v, m = _cuda(*make_case(b, h, hk, sq, sk, d, dtype, kind, seed=61))
+    out, lse, _ = run_cabi(q, k, v, m, want_lse=True, num_splits=splits, no_unit_cut=1)
+    out1, lse1, _ = run_cabi(q, k, v, m, want_lse=True, num_splits=splits, no_unit_cut=1, no_head_pairs=1)
+    if splits == 1 or h // hk * sq <= 128:      # (else one run merges slots in the CTA and the other does not)
+        assert torch.equal(out, out1) and torch.equal(lse, lse1)
+    auto, _, _ = run_cabi(q, k, v, m)
+    for o in (out, auto):
+        check_against_oracle(o, q, k, v, m, f"packed{case}")
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case", [
+    # b, h, hk, sq, sk, d, rule; more than 24 key blocks and fewer units than SMs
+    (1, 4, 4, 1, 3201, 128, dict(valid_lens=[2900])),             # one row, two key ranges per CTA
+    (3, 8, 2, 1, 5000, 64, dict(causal=True, valid_lens=[5000, 130, 0])),   # packed; fewer visible blocks than shares
+    (1, 4, 2, 128, 8192, 128, dict(causal=True)),
+    (2, 4, 1, 50, 4099, 128, dict(causal=True)),                  # 200 packed rows: cut in pieces
+    (1, 4, 2, 300, 4096, 128, dict(causal=True)),                 # pairs of heads, cut in pieces
+    (2, 2, 2, 520, 3300, 64, dict(valid_lens=[3300, 1])),         # pieces of one block, and of none
+    (1, 2, 2, 260, 9000, 128, dict(causal=True, window=4000)),    # a window wide enough to cut
+])
+def test_rule_attention_over_long_keys_is_split(dtype, case):
+    """Under a rule, few units over many keys are split over the GPU.  The partials are merged in
+    fp32, so the result stays within one rounding of the output type (2^-8 or 2^-11 relative, of
+    values below 2) of the single pass."""
+    from custom_ops_b200.masks import rule_attention, rule_mask
+    b, h, hk, sq, sk, d, rule = case
+    q, k, v, _ = make_case(b, h, hk, sq, sk, d, dtype, "zero", seed=67)
+    q, k, v = _cuda(q, k, v)
+    lens = torch.tensor(rule["valid_lens"], dtype=torch.int32) if "valid_lens" in rule else None
+    kw = dict(causal=rule.get("causal", False), window=rule.get("window", 0), valid_lens=lens)
+    m = rule_mask(b, sq, sk, dtype=dtype, **kw)
+    want, want_lse, _ = run_cabi(q, k, v, m, num_splits=1, no_unit_cut=1, want_lse=True)
+    args = _cabi.make_args(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), mask=0, out=q.data_ptr(), batch=b, heads=h,
+                           heads_k=hk, seqlen_q=sq, seqlen_k=sk, head_dim=d,
+                           dtype=_cabi.BF16 if dtype == torch.bfloat16 else _cabi.FP16)
+    assert _cabi.rule_workspace_bytes(args, kw["window"]) > _cabi.RULE_WORKSPACE_BYTES
+    for _ in range(2):                                            # (the second run finds the first one's scratch)
+        got, got_lse = rule_attention(q, k, v, return_lse=True, **kw)
+        torch.cuda.synchronize()
+        assert (got.float() - want.float()).abs().max().item() <= (2 ** -7 if dtype == torch.bfloat16 else 2 ** -10)
+        assert torch.equal(torch.isneginf(got_lse), torch.isneginf(want_lse))
+        fin = torch.isfinite(want_lse)
+        assert (got_lse[fin] - want_lse[fin]).abs().max().item() <= 1e-4
+    check_against_oracle(got, q, k, v, m[..., :sk].contiguous(), f"rule_split{case}")
+    assert _cabi.device_status(0, clear=True) == 0
