@@ -326,7 +326,10 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         sts32(wait_limit, p.wait_kcycles);
     }
     __syncthreads();
-    if (lds32(bail_word) != 0) return;
+    if (lds32(bail_word) != 0) {
+        pdl_wait_prior_grid();        // (no launch may count as finished before the one ahead of it)
+        return;
+    }
 
     // The CTA is persistent in pair mode: it takes units blockIdx.x, blockIdx.x + gridDim.x, ...
     // and every role keeps running counters for its barrier phases, so the producers and the
@@ -349,8 +352,8 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
     // unit-scheduler role below).  The board is plain shared memory: the first unit of a CTA -
     // always unit blockIdx.x, whole - is decoded before the set-up barrier, under the tensor
     // memory allocation and the mbarrier initialisation of the other warps, and only its
-    // arrival on the "full" mbarrier waits for that barrier.  (Not with a skip list: the block
-    // flags are only valid once the pre-pass kernel has finished.)
+    // arrival on the "full" mbarrier waits for that barrier.  (Not with a skip list or a rule: the
+    // block flags and the valid lengths may only be read once the kernel before has finished.)
     auto publish_unit = [&](int k, int unit, int part, int part_begin, int part_n, int peer_last) {
         int rest = unit;
         const int sgroup = rest % p.split_groups;
@@ -450,7 +453,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
     // (The first unit of a CTA is unit blockIdx.x, whole, and can be decoded before the set-up
     // barrier - unless the launch has fewer units than CTAs, where every unit is cut in pieces.)
     const bool first_unit_whole = !(p.cut_units != 0 && p.total_units < static_cast<int>(gridDim.x));
-    if (!LIST && first_unit_whole && warp == 11)
+    if (!LIST && !RULE && first_unit_whole && warp == 11)
         publish_unit(0, static_cast<int>(blockIdx.x), kPartWhole, 0, p.kv_blocks, 0);
 
     if (warp == kTmaWarp && lane == 0) {
@@ -508,6 +511,12 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         if (warp == kTmaWarp) {
             // -------------------------------------------------------------- Q/K/V producer
             if (lane == 0) {
+                // Every launch is chained to the kernel before it (programmatic dependent launch), which
+                // may still be writing q, k and v, or reading what this launch will overwrite.  All of
+                // the CTA's loads of operands, and so everything it stores, come behind this wait or
+                // the mask producer's or the scheduler's; set-up and the softmax warps' first pass
+                // through their code run under the tail of the kernel before.
+                pdl_wait_prior_grid();
                 Ring ring;                      // next ring slot to fill, over all units
                 int in_flight = 0;              // fills issued (capped), for the drain below
                 uint32_t q_phase[2] = {1u, 1u}; // parity that says "Q tile t may be overwritten"
@@ -599,9 +608,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         } else if (warp == kMaskWarp) {
             // -------------------------------------------------------------- mask producer
             if (lane == 0) {
-                // The mask may be a re-pitched copy written by the kernel launched just before
-                // this one (chained with programmatic dependent launch): wait for it here, so
-                // everything that does not need the mask has already started.
+                // (the mask may be a re-pitched copy written by the kernel launched just before)
                 pdl_wait_prior_grid();
                 // Panel i = slot * 2 + half.  A slot's panels follow that slot's own key blocks.
                 uint32_t ph[4] = {0u, 0u, 0u, 0u};      // phase of panel i's next load
@@ -660,7 +667,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
             // compacts the unit's block flags - a pre-pass kernel marked the key blocks whose
             // mask is -inf for all 256 rows of a pair - into the list of blocks to visit.
             // Skipping such a block is exact: all of its weights are 0.
-            if constexpr (LIST) pdl_wait_prior_grid();     // the flags come from the pre-pass kernel
+            if constexpr (LIST || RULE) pdl_wait_prior_grid();     // flags, valid lengths, unit counter
             // Which unit comes next: a CTA starts with unit blockIdx.x; after that it takes every
             // gridDim.x-th one, or - with tile skipping, where units differ in length - the next
             // one nobody has taken yet, from a counter the pre-pass kernel reset.
@@ -710,7 +717,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                     }
                     break;
                 }
-                if (LIST || k > 0 || !first_unit_whole) publish_unit(k, unit, part, part_begin, part_n, peer_last);
+                if (LIST || RULE || k > 0 || !first_unit_whole) publish_unit(k, unit, part, part_begin, part_n, peer_last);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_unit_full + 8 * (k & 1));    // release: board and list visible
             }
@@ -1428,6 +1435,7 @@ fa_mask_combine_kernel(const float* __restrict__ o_parts, const float* __restric
     const long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     // When chained behind the attention kernel with programmatic dependent launch, the
     // partials are only valid after this returns; otherwise it returns at once.
+    pdl_launch_dependents();
     pdl_wait_prior_grid();
     const bool peers = px.parts != nullptr;
     if (peers) {
@@ -1579,8 +1587,8 @@ fa_mask_classify_kernel(const uint16_t* __restrict__ mask, long long bs, long lo
                         uint32_t neg_inf2, unsigned char* __restrict__ flags, int* hint,
                         unsigned int* unit_counter, int region_rows) {
     const int nt = blockIdx.x, mp = blockIdx.y, b = blockIdx.z;
-    pdl_wait_prior_grid();                          // a re-pitch kernel may have written the mask
     pdl_launch_dependents();
+    pdl_wait_prior_grid();                          // the kernel before may have written the mask
     // the attention kernel behind this one hands out its units from this counter
     if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) *unit_counter = 0u;
     const int vec = threadIdx.x & 15;               // 16 vectors of 8 keys per 128-key row piece
@@ -1654,6 +1662,7 @@ __global__ void __launch_bounds__(256)
 fa_mask_repitch_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int Sq, int Sk,
                        int pitch, long long src_bs, long long src_rs) {
     pdl_launch_dependents();
+    pdl_wait_prior_grid();
     const long long r = blockIdx.x;                  // b * Sq + row
     const int b = static_cast<int>(r / Sq);
     const int row = static_cast<int>(r % Sq);
@@ -1708,12 +1717,21 @@ fa_mask_repitch_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ 
     }
 }
 
+// The counter the CTAs of a rule launch take their units from starts at 0.
+__global__ void fa_zero_counter_kernel(unsigned int* counter) {
+    pdl_launch_dependents();
+    pdl_wait_prior_grid();
+    if (threadIdx.x == 0) *counter = 0u;
+}
+
 // ---------------------------------------------------------------------------------
 // Mask from rules (padding / causal / sliding window): one 16-byte vector per thread.
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
 fa_mask_build_kernel(uint16_t* __restrict__ mask, int Sq, int Sk, int pitch, uint32_t neg_inf16, int causal,
                      int window, const int* __restrict__ valid_lens) {
+    pdl_launch_dependents();
+    pdl_wait_prior_grid();
     const long long r = blockIdx.x;                   // b * Sq + i
     const int b = static_cast<int>(r / Sq);
     const int i = static_cast<int>(r % Sq);
@@ -2062,6 +2080,30 @@ static int encode_map(CUtensorMap* tm, const void* ptr, int dtype, int planes, i
     return r == CUDA_SUCCESS ? FA_SM100_OK : FA_SM100_ERR_CUDA;
 }
 
+// Every kernel is launched chained to the kernel before it in the stream: its CTAs become resident
+// as soon as all of that kernel's CTAs have started and SMs are free, run what needs no memory of
+// the caller's, and wait (griddepcontrol.wait) for the kernel before to finish and its writes to be
+// visible.  Behind a kernel that does not announce its dependents the wait ends with that kernel.
+// Every kernel here executes the wait, so "the kernel before has finished" covers all before it.
+// Back to back calls, before and after: 1.3 MB of operands 12.3 -> 8.2 us, a decode step over 8 x 4096
+// keys 26.6 -> 22.1 us, Split-KV over 32768 keys 73.7 -> 69.8 us.
+template <typename Kern, typename... Args>
+static bool launch_chained(Kern kern, dim3 grid, int threads, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaLaunchKernelEx(&cfg, kern, args...) != cudaSuccess) return false;
+    ++g_launches;
+    return true;
+}
+
 // The four tensor maps depend only on pointers, shapes, pitches and dtype, not on data, and
 // callers tend to come back with the same buffers (a layer called every step, a benchmark
 // loop), so the last few sets are kept: encoding them costs several microseconds of host
@@ -2113,7 +2155,7 @@ static int get_maps(const MapKey& key, CUtensorMap* tq, CUtensorMap* tk, CUtenso
 template <int D, bool BF16, bool LIST, bool RULE, bool PACK>
 static int launch_fwd(DeviceInfo* dev, const CUtensorMap& tq, const CUtensorMap& tk,
                       const CUtensorMap& tv, const CUtensorMap& tm, const KParams& kp, dim3 grid,
-                      cudaStream_t stream, bool chained) {
+                      cudaStream_t stream) {
     auto kern = fa_mask_fwd_kernel<D, BF16, LIST, RULE, PACK>;
     const int slot = (D == 128 ? 0 : 1) + (BF16 ? 0 : 2) + (PACK ? 4 : 0) + (RULE ? 16 : LIST ? 8 : 0);
     if (!dev->attr_set[slot]) {
@@ -2133,33 +2175,13 @@ static int launch_fwd(DeviceInfo* dev, const CUtensorMap& tq, const CUtensorMap&
         }
         dev->attr_set[slot] = true;
     }
-    if (chained) {
-        // behind a pre-pass kernel: start this kernel's prologue under that kernel's tail
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(kThreads);
-        cfg.dynamicSmemBytes = Cfg<D>::kSmemBytes;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tm, kp) != cudaSuccess) {
-            return cuda_failed(__LINE__);
-        }
-        ++g_launches;
-        return FA_SM100_OK;
-    }
-    kern<<<grid, kThreads, Cfg<D>::kSmemBytes, stream>>>(tq, tk, tv, tm, kp);
-    if (cudaPeekAtLastError() != cudaSuccess) return cuda_failed(__LINE__);
-    ++g_launches;
+    if (!launch_chained(kern, grid, kThreads, Cfg<D>::kSmemBytes, stream, tq, tk, tv, tm, kp)) return cuda_failed(__LINE__);
     return FA_SM100_OK;
 }
 
 static int launch_combine(const float* o_parts, const float* lse_parts, void* out, float* lse_out,
                           int parts, long long rows, int d, int dtype, int out_fp32,
-                          cudaStream_t stream, bool chained = false, long long o_part_stride = 0,
+                          cudaStream_t stream, long long o_part_stride = 0,
                           long long lse_part_stride = 0, const PeerExchange* peer = nullptr) {
     if (rows <= 0) return FA_SM100_OK;
     PeerExchange px;
@@ -2170,43 +2192,13 @@ static int launch_combine(const float* o_parts, const float* lse_parts, void* ou
     if (lse_part_stride == 0) lse_part_stride = rows;
     const int warps = 8;
     const unsigned blocks = static_cast<unsigned>((rows + warps - 1) / warps);
-    if (chained) {
-        // Programmatic dependent launch behind the attention kernel: the launch latency
-        // hides under that kernel's tail; the merge kernel waits on the grid dependency
-        // before it reads a partial.
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(warps * 32);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        const int is_bf16 = dtype == FA_SM100_BF16;
-        cudaError_t e = (d == 128)
-            ? cudaLaunchKernelEx(&cfg, fa_mask_combine_kernel<128>, o_parts, lse_parts, out, lse_out,
-                                 parts, rows, is_bf16, out_fp32, o_part_stride, lse_part_stride, px)
-            : cudaLaunchKernelEx(&cfg, fa_mask_combine_kernel<64>, o_parts, lse_parts, out, lse_out,
-                                 parts, rows, is_bf16, out_fp32, o_part_stride, lse_part_stride, px);
-        if (e != cudaSuccess) {
-            return cuda_failed(__LINE__);
-        }
-        ++g_launches;
-        return FA_SM100_OK;
-    }
-    if (d == 128)
-        fa_mask_combine_kernel<128><<<blocks, warps * 32, 0, stream>>>(
-            o_parts, lse_parts, out, lse_out, parts, rows, dtype == FA_SM100_BF16, out_fp32,
-            o_part_stride, lse_part_stride, px);
-    else
-        fa_mask_combine_kernel<64><<<blocks, warps * 32, 0, stream>>>(
-            o_parts, lse_parts, out, lse_out, parts, rows, dtype == FA_SM100_BF16, out_fp32,
-            o_part_stride, lse_part_stride, px);
-    if (cudaPeekAtLastError() != cudaSuccess) return cuda_failed(__LINE__);
-    ++g_launches;
-    return FA_SM100_OK;
+    const int is_bf16 = dtype == FA_SM100_BF16;
+    const bool ok = d == 128
+        ? launch_chained(fa_mask_combine_kernel<128>, dim3(blocks), warps * 32, 0, stream, o_parts, lse_parts, out, lse_out,
+                         parts, rows, is_bf16, out_fp32, o_part_stride, lse_part_stride, px)
+        : launch_chained(fa_mask_combine_kernel<64>, dim3(blocks), warps * 32, 0, stream, o_parts, lse_parts, out, lse_out,
+                         parts, rows, is_bf16, out_fp32, o_part_stride, lse_part_stride, px);
+    return ok ? FA_SM100_OK : cuda_failed(__LINE__);
 }
 
 static int status_pointer(DeviceInfo* dev) {
@@ -2485,10 +2477,10 @@ static void flag_cache_read(int device, int slot, cudaStream_t stream) {
 template <int D, bool BF16, bool PACK>
 static int launch_variant(bool list, bool rule, DeviceInfo* dev, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tm, const KParams& kp, dim3 grid,
-                          cudaStream_t stream, bool chained) {
-    if (rule) return launch_fwd<D, BF16, false, true, PACK>(dev, tq, tk, tv, tm, kp, grid, stream, chained);
-    if (list) return launch_fwd<D, BF16, true, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream, chained);
-    return launch_fwd<D, BF16, false, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream, chained);
+                          cudaStream_t stream) {
+    if (rule) return launch_fwd<D, BF16, false, true, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
+    if (list) return launch_fwd<D, BF16, true, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
+    return launch_fwd<D, BF16, false, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
 }
 
 static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_bytes,
@@ -2555,10 +2547,9 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
         const int pitch = (a->seqlen_k + 7) & ~7;
         uint16_t* dst = reinterpret_cast<uint16_t*>(ws);
         const unsigned blocks = static_cast<unsigned>(a->batch) * a->seqlen_q;
-        fa_mask_repitch_kernel<<<blocks, 256, 0, stream>>>(
-            mask_ptr, dst, a->seqlen_q, a->seqlen_k, pitch, mask_bs, mask_rs);
-        if (cudaPeekAtLastError() != cudaSuccess) return cuda_failed(__LINE__);
-        ++g_launches;
+        if (!launch_chained(fa_mask_repitch_kernel, dim3(blocks), 256, 0, stream, mask_ptr, dst, a->seqlen_q, a->seqlen_k,
+                            pitch, mask_bs, mask_rs))
+            return cuda_failed(__LINE__);
         mask_ptr = dst;
         mask_bs = static_cast<long long>(a->seqlen_q) * pitch;
         mask_rs = pitch;
@@ -2591,20 +2582,9 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
         unsigned int* unit_counter = ws_unit_counter;
         const dim3 cgrid(plan.kv_blocks, regions, a->batch);
         const uint32_t ninf = a->dtype == FA_SM100_BF16 ? 0xFF80FF80u : 0xFC00FC00u;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = cgrid;
-        cfg.blockDim = dim3(256);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = plan.mask_repitched ? 1 : 0;      // chained behind the re-pitch kernel
-        if (cudaLaunchKernelEx(&cfg, fa_mask_classify_kernel, mask_ptr, mask_bs, mask_rs, a->seqlen_q,
-                               a->seqlen_k, ninf, flags, hint_counter, unit_counter, region_rows) != cudaSuccess) {
+        if (!launch_chained(fa_mask_classify_kernel, cgrid, 256, 0, stream, mask_ptr, mask_bs, mask_rs, a->seqlen_q,
+                            a->seqlen_k, ninf, flags, hint_counter, unit_counter, region_rows))
             return cuda_failed(__LINE__);
-        }
-        ++g_launches;
         kp.block_flags = flags;
         kp.unit_counter = unit_counter;
         if (cache == kFlagsFill) flag_cache_filled(a->device, flag_slot, stream);
@@ -2648,7 +2628,8 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
         if (rule->counter != nullptr && kp.cut_units == 0 && !plan.dual_split && kp.total_units > plan.grid_x) {
             // (only where a CTA takes more than its first unit; a compare-and-swap counter that tolerates any content was measured first: with 148
             // CTAs drawing in waves its retries are quadratic and cost 100 us per launch)
-            if (cudaMemsetAsync(rule->counter, 0, sizeof(unsigned int), stream) != cudaSuccess) return cuda_failed(__LINE__);
+            // (a kernel and not a memset: a memset between two kernels cannot be chained)
+            if (!launch_chained(fa_zero_counter_kernel, dim3(1), 32, 0, stream, rule->counter)) return cuda_failed(__LINE__);
             kp.unit_counter = rule->counter;
         }
     }
@@ -2672,7 +2653,6 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     if ((rc = get_maps(key, &tq, &tk, &tv, &tm)) != FA_SM100_OK) return rc;
 
     const dim3 grid(plan.grid_x, plan.grid_y, plan.grid_z);
-    const bool chained = plan.mask_repitched || run_classify;
     const bool bf16 = a->dtype == FA_SM100_BF16;
     const bool list = kp.block_flags != nullptr;
     // (a rule launch has no skip list and nothing to re-pitch: fa_mask_fwd_sm100_rule sees to that)
@@ -2680,8 +2660,8 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     auto launch = [&](auto head_dim, auto is_bf16) {
         constexpr int kD = decltype(head_dim)::value;
         constexpr bool kBf16 = decltype(is_bf16)::value;
-        return pack_kernel ? launch_variant<kD, kBf16, true>(list, rule != nullptr, dev, tq, tk, tv, tm, kp, grid, stream, chained)
-                           : launch_variant<kD, kBf16, false>(list, rule != nullptr, dev, tq, tk, tv, tm, kp, grid, stream, chained);
+        return pack_kernel ? launch_variant<kD, kBf16, true>(list, rule != nullptr, dev, tq, tk, tv, tm, kp, grid, stream)
+                           : launch_variant<kD, kBf16, false>(list, rule != nullptr, dev, tq, tk, tv, tm, kp, grid, stream);
     };
     if (d == 128) rc = bf16 ? launch(std::integral_constant<int, 128>{}, std::true_type{})
                             : launch(std::integral_constant<int, 128>{}, std::false_type{});
@@ -2692,7 +2672,7 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     if (plan.num_splits > 1)
         rc = launch_combine(o_part, lse_part, a->out, a->lse,
                             plan.dual_split ? ceil_div(plan.num_splits, 2) : plan.num_splits, rows, d,
-                            a->dtype, a->out_fp32, stream, /*chained=*/true);
+                            a->dtype, a->out_fp32, stream);
     return rc;
 }
 
@@ -2811,7 +2791,7 @@ int fa_mask_fwd_sm100_combine_packed(const float* packed, int64_t part_stride, v
         return fa_sm100::cuda_failed(__LINE__);
     }
     return fa_sm100::launch_combine(packed, packed + rows * head_dim, out, lse_out, num_parts, rows, head_dim,
-                                    dtype, out_fp32, static_cast<cudaStream_t>(stream), false, part_stride,
+                                    dtype, out_fp32, static_cast<cudaStream_t>(stream), part_stride,
                                     part_stride);
 }
 
@@ -2847,7 +2827,7 @@ int fa_mask_fwd_sm100_combine_peers(const void* part_table, int64_t part_offset,
     px.wait_kcycles = fa_sm100::kMaxWaitKcycles;
     px.status = dev->status_ptr;
     return fa_sm100::launch_combine(nullptr, nullptr, out, lse_out, world, rows, head_dim, dtype, out_fp32,
-                                    static_cast<cudaStream_t>(stream), false, 0, 0, &px);
+                                    static_cast<cudaStream_t>(stream), 0, 0, &px);
 }
 
 int fa_mask_fwd_sm100_device_status(int32_t device, uint32_t* status, int32_t clear) {
@@ -2893,11 +2873,10 @@ int fa_mask_build_sm100(void* mask, int32_t batch, int32_t seqlen_q, int32_t seq
     const unsigned vec_blocks = static_cast<unsigned>((pitch + 8 * 256 - 1) / (8 * 256));
     if (vec_blocks > 65535u) return FA_SM100_ERR_SHAPE;
     const uint32_t neg = dtype == FA_SM100_BF16 ? 0xFF80u : 0xFC00u;
-    fa_sm100::fa_mask_build_kernel<<<dim3(static_cast<unsigned>(rows), vec_blocks), 256, 0,
-                                     static_cast<cudaStream_t>(stream)>>>(
-        static_cast<uint16_t*>(mask), seqlen_q, seqlen_k, pitch, neg, causal, window, valid_lens);
-    if (cudaPeekAtLastError() != cudaSuccess) return fa_sm100::cuda_failed(__LINE__);
-    ++fa_sm100::g_launches;
+    if (!fa_sm100::launch_chained(fa_sm100::fa_mask_build_kernel, dim3(static_cast<unsigned>(rows), vec_blocks), 256, 0,
+                                  static_cast<cudaStream_t>(stream), static_cast<uint16_t*>(mask), seqlen_q, seqlen_k,
+                                  pitch, neg, causal, window, static_cast<const int*>(valid_lens)))
+        return fa_sm100::cuda_failed(__LINE__);
     return FA_SM100_OK;
 }
 

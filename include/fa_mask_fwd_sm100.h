@@ -213,8 +213,7 @@ int fa_mask_fwd_sm100_static_scratch(const FaMaskFwdArgs* args, void* stream);
  *       too few units would leave SMs idle (fp32 partials, merged; the rounding of the merge is then
  *       the only difference);
  *   FA_SM100_RULE_WORKSPACE_BYTES: one pass; the counter the CTAs take their units from (units differ
- *       in length under a rule; the call zeroes it on the stream with a cudaMemsetAsync ahead of the
- *       kernel);
+ *       in length under a rule; the call zeroes it on the stream ahead of the kernel);
  *   NULL: one pass, every CTA takes a fixed share of the units (slower where the lengths differ much).
  * The reference has no such operator. */
 #define FA_SM100_RULE_WORKSPACE_BYTES 16
