@@ -1285,15 +1285,6 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                     }
                     if (!alive) break;
                 }
-                // the whole row is read from tensor memory with one load and one wait
-                uint32_t o[D];
-                if (!empty) {
-                    if constexpr (D == 128) tmem_ld128(tO, o);
-                    else tmem_ld64(tO, o);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < D; ++i) o[i] = 0u;
-                }
                 // where the row goes: the output, a Split-KV partial, or this CTA's cut partial
                 const long long grow = (static_cast<long long>(u_b) * p.H + u_h) * p.Sq + row;
                 float* o32 = nullptr;
@@ -1317,52 +1308,68 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                     if (row_ok && p.lse != nullptr) p.lse[grow] = lse_val;
                 }
                 uint16_t* o16 = static_cast<uint16_t*>(p.out) + grow * D;
+                if (empty) {
+                    // no key block was visited: nothing is in the O columns yet, the result is 0
+#pragma unroll 1
+                    for (int c = 0; c < D; ++c) tmem_st1(tO + c, 0u);
+                    tmem_wait_st();
+                }
+                // Rolled on purpose: this code runs once per unit, from no instruction cache, so every
+                // line of it costs a miss.  Unrolled over the whole row the epilogue made calls of short
+                // units slower (4 x 2048 x 2048 under a window of 512, as a rule 63.4 us against 60.9, as
+                // a mask tensor 78.1 against 75.7; 16 key blocks per unit: 174.7 against 172.5).
                 if (wide) {
                     // quad-transposed, line-sized stores (see quad_transpose)
                     if (o32 != nullptr) {
-#pragma unroll
+#pragma unroll 1
                         for (int c = 0; c < D / 32; ++c) {
                             uint32_t w[32];
+                            __syncwarp();
+                            tmem_ld32(tO + c * 32, w);
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(__uint_as_float(o[c * 32 + i]) * inv);
+                            for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(__uint_as_float(w[i]) * inv);
                             quad_transpose(w, lane);
                             quad_store(w, lane, reinterpret_cast<char*>(o32 + c * 32), static_cast<long long>(D) * 4,
                                        rows_left);
                         }
                     } else {
-#pragma unroll
+#pragma unroll 1
                         for (int c = 0; c < D / 64; ++c) {
-                            uint32_t w[32];
+                            uint32_t o[64], w[32];
+                            __syncwarp();
+                            tmem_ld64(tO + c * 64, o);
 #pragma unroll
                             for (int i = 0; i < 32; ++i)
-                                w[i] = pack2<BF16>(__uint_as_float(o[c * 64 + 2 * i]) * inv,
-                                                   __uint_as_float(o[c * 64 + 2 * i + 1]) * inv);
+                                w[i] = pack2<BF16>(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
                             quad_transpose(w, lane);
                             quad_store(w, lane, reinterpret_cast<char*>(o16 + c * 64), static_cast<long long>(D) * 2,
                                        rows_left);
                         }
                     }
-                } else if (row_ok) {
+                } else {
                     // an output that is only 16-byte aligned: each thread stores its own row
-                    if (o32 != nullptr) {
+#pragma unroll 1
+                    for (int c = 0; c < D / 32; ++c) {
+                        uint32_t o[32];
+                        __syncwarp();
+                        tmem_ld32(tO + c * 32, o);
+                        if (!row_ok) {
+                        } else if (o32 != nullptr) {
 #pragma unroll
-                        for (int i = 0; i < D; i += 4) {
-                            float4 f;
-                            f.x = __uint_as_float(o[i]) * inv;
-                            f.y = __uint_as_float(o[i + 1]) * inv;
-                            f.z = __uint_as_float(o[i + 2]) * inv;
-                            f.w = __uint_as_float(o[i + 3]) * inv;
-                            *reinterpret_cast<float4*>(o32 + i) = f;
-                        }
-                    } else {
+                            for (int i = 0; i < 32; i += 4)
+                                *reinterpret_cast<float4*>(o32 + c * 32 + i) =
+                                    make_float4(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv,
+                                                __uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                        } else {
 #pragma unroll
-                        for (int i = 0; i < D; i += 8) {
-                            uint4 uu;
-                            uu.x = pack2<BF16>(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
-                            uu.y = pack2<BF16>(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
-                            uu.z = pack2<BF16>(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
-                            uu.w = pack2<BF16>(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
-                            *reinterpret_cast<uint4*>(o16 + i) = uu;
+                            for (int i = 0; i < 32; i += 8) {
+                                uint4 uu;
+                                uu.x = pack2<BF16>(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                                uu.y = pack2<BF16>(__uint_as_float(o[i + 2]) * inv, __uint_as_float(o[i + 3]) * inv);
+                                uu.z = pack2<BF16>(__uint_as_float(o[i + 4]) * inv, __uint_as_float(o[i + 5]) * inv);
+                                uu.w = pack2<BF16>(__uint_as_float(o[i + 6]) * inv, __uint_as_float(o[i + 7]) * inv);
+                                *reinterpret_cast<uint4*>(o16 + c * 32 + i) = uu;
+                            }
                         }
                     }
                 }
