@@ -512,10 +512,10 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
             // -------------------------------------------------------------- Q/K/V producer
             if (lane == 0) {
                 // Every launch is chained to the kernel before it (programmatic dependent launch), which
-                // may still be writing q, k and v, or reading what this launch will overwrite.  All of
-                // the CTA's loads of operands, and so everything it stores, come behind this wait or
-                // the mask producer's or the scheduler's; set-up and the softmax warps' first pass
-                // through their code run under the tail of the kernel before.
+                // may still be writing q, k and v, or reading what this launch will overwrite.  Every
+                // role waits for it before its first bounded wait, so that those limits count this
+                // launch's own time only; set-up and the softmax warps' first pass through their code
+                // run under the tail of the kernel before.
                 pdl_wait_prior_grid();
                 Ring ring;                      // next ring slot to fill, over all units
                 int in_flight = 0;              // fills issued (capped), for the drain below
@@ -667,7 +667,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
             // compacts the unit's block flags - a pre-pass kernel marked the key blocks whose
             // mask is -inf for all 256 rows of a pair - into the list of blocks to visit.
             // Skipping such a block is exact: all of its weights are 0.
-            if constexpr (LIST || RULE) pdl_wait_prior_grid();     // flags, valid lengths, unit counter
+            pdl_wait_prior_grid();     // flags, valid lengths, unit counter
             // Which unit comes next: a CTA starts with unit blockIdx.x; after that it takes every
             // gridDim.x-th one, or - with tile skipping, where units differ in length - the next
             // one nobody has taken yet, from a counter the pre-pass kernel reset.
@@ -724,6 +724,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         } else if (warp == kMmaWarp) {
             // -------------------------------------------------------------- MMA issuer
             if (lane == 0) {
+                pdl_wait_prior_grid();
                 constexpr uint32_t idesc_s = make_idesc(BF16, false, kBlockM, kBlockN);
                 constexpr uint32_t idesc_o = make_idesc(BF16, true, kBlockM, D);
                 const uint32_t tS0 = tmem_base;
@@ -1123,7 +1124,10 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 gstep += dummy ? 0 : 1;
             }
             if (!alive) break;
-            if (warm) continue;
+            if (warm) {
+                pdl_wait_prior_grid();
+                continue;
+            }
             // the rest of the unit's description is read from the board only now, so that it
             // holds no registers during the loop above
             const int row = ui_get(ui, kUiSlot + 4 * t + kUiRow0) + row_in_tile;
