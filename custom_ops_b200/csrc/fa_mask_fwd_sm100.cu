@@ -184,6 +184,10 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // merging CTA is the one that is dispatched last: whatever it waits for was written by CTAs
 // that are already resident or finished, also when another kernel holds part of the GPU.  (Equal shares of ALL steps, or of the last round's, were
 // measured and lose: the partial traffic of 148 CTAs at once costs more than the idle SMs.)
+// Block flags of the pre-pass (0: every key of the block is hidden for all rows of the region), and
+// the mark a visit list carries on the blocks whose mask is zero throughout.
+enum : unsigned char { kFlagMixed = 1, kFlagPlain = 2 };
+constexpr uint32_t kListPlain = 0x8000u;
 enum : int { kPartWhole = 0, kPartTail = 1, kPartHead = 2 };
 
 // Unit board: what the scheduler warp publishes about one unit of work, a (split group,
@@ -373,7 +377,9 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 const int jj = base_j + lane;
                 const bool need = jj < p.kv_blocks && fl[jj] != 0;
                 const unsigned ballot = __ballot_sync(0xffffffffu, need);
-                if (need) sts16(lst + 2 * (count + __popc(ballot & ((1u << lane) - 1u))), static_cast<uint32_t>(jj));
+                if (need)
+                    sts16(lst + 2 * (count + __popc(ballot & ((1u << lane) - 1u))),
+                          static_cast<uint32_t>(jj) | (fl[jj] == kFlagPlain ? kListPlain : 0u));
                 count += __popc(ballot);
             }
         }
@@ -569,7 +575,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                         if (!dual) {
                             // shared by both slots: K_0, V_0, K_1, V_1, ...
                             for (int j = 0; ok && j < n0; ++j) {
-                                const int blk = LIST ? static_cast<int>(lds16(lst + 2 * j)) : begin0 + j;
+                                const int blk = LIST ? static_cast<int>(lds16(lst + 2 * j) & ~kListPlain) : begin0 + j;
                                 ok = fill(false, blk) && fill(true, blk);
                             }
                         } else {
@@ -631,6 +637,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                             if (!ok || j >= n_of[t]) continue;
                             if (t == 1 && p.head_pairs) continue;      // slot 1 reads slot 0's panels
                             const int blk = LIST ? static_cast<int>(lds16(lst + 2 * j)) : begin_of[t] + j;
+                            if (LIST && (blk & kListPlain)) continue;      // nothing to add: no tile wanted
 #pragma unroll
                             for (int hf = 0; hf < 2; ++hf) {
                                 const int i = 2 * t + hf;
@@ -906,6 +913,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         const float2 scale2 = make_float2(p.scale, p.scale);
 
         int gstep = 0;               // key-block steps of this slot so far, over all units
+        [[maybe_unused]] int mstep = 0;   // LIST: those of them that had a mask tile
         int o_uses = 0;              // units of this slot that waited for their final O
         bool alive = true;
         // The body of a key-block step is some 15 KB of straight-line code, and a launch finds it
@@ -959,7 +967,10 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
             asm volatile("" : "+r"(j));  // (opaque: the first pass must stay inside the loop's code)
             for (; j < n_t; ++j) {
                 const bool dummy = j < 0;
-                const int col0 = (LIST ? static_cast<int>(lds16(lst + 2 * j)) : begin_t + j) * kBlockN;
+                const int entry = LIST ? static_cast<int>(lds16(lst + 2 * j)) : begin_t + j;
+                // LIST: a block whose mask is zero throughout has no mask tile in shared memory
+                const bool plain_mask = LIST && !dummy && (entry & kListPlain) != 0;
+                const int col0 = (LIST ? entry & ~static_cast<int>(kListPlain) : entry) * kBlockN;
                 const bool tail = !dummy && (col0 + kBlockN) > p.Sk;
                 const uint32_t par = (gstep & 1) ^ (dummy ? 1u : 0u);
 
@@ -969,9 +980,10 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 // latency falls into time the thread would spend waiting anyway, so that nothing
                 // but the wake-up from the score barrier stands between S and the first load.
                 bool ok = true;
-                if constexpr (!RULE) {
-                    ok = mbar_wait(dummy ? bar_scratch : bar_m_full + 8 * (2 * mt), par, abort_flag, p.status, kStSoftmaxMask);
-                    ok = mbar_wait(dummy ? bar_scratch : bar_m_full + 8 * (2 * mt + 1), par, abort_flag, p.status, kStSoftmaxMask) && ok;
+                if (!RULE && !plain_mask) {
+                    const uint32_t m_par = LIST ? (mstep & 1) ^ (dummy ? 1u : 0u) : par;
+                    ok = mbar_wait(dummy ? bar_scratch : bar_m_full + 8 * (2 * mt), m_par, abort_flag, p.status, kStSoftmaxMask);
+                    ok = mbar_wait(dummy ? bar_scratch : bar_m_full + 8 * (2 * mt + 1), m_par, abort_flag, p.status, kStSoftmaxMask) && ok;
                 }
                 ok = mbar_wait(dummy ? bar_scratch : bar_s, par, abort_flag, p.status, kStSoftmaxS) && ok;
                 if (!__all_sync(0xffffffffu, ok)) { alive = false; break; }
@@ -993,6 +1005,20 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 tmem_ld128(tS, sreg);
                 float2 x[kBlockN / 2];
                 float mt0 = -INFINITY, mt1 = -INFINITY;
+                auto scale_only = [&]() {
+                    const float2 zero2 = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int i = 0; i < kBlockN; i += 4) {
+                        const float2 xa = __ffma2_rn(
+                            make_float2(__uint_as_float(sreg[i]), __uint_as_float(sreg[i + 1])), scale2, zero2);
+                        const float2 xb = __ffma2_rn(
+                            make_float2(__uint_as_float(sreg[i + 2]), __uint_as_float(sreg[i + 3])), scale2, zero2);
+                        x[i / 2] = xa;
+                        x[i / 2 + 1] = xb;
+                        mt0 = max3(mt0, xa.x, xb.x);
+                        mt1 = max3(mt1, xa.y, xb.y);
+                    }
+                };
                 if constexpr (RULE) {
                     // No mask tile: the row sees the keys (rule_lo, rule_hi].  A block that every
                     // row of the warp sees entirely needs nothing but the scale; otherwise the
@@ -1001,18 +1027,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                     const int rel_lo = rule_lo - col0, rel_hi = rule_hi - col0;
                     const bool plain = __all_sync(0xffffffffu, rel_lo < 0 && rel_hi >= kBlockN - 1) && !dummy;
                     if (plain) {
-                        const float2 zero2 = make_float2(0.f, 0.f);
-#pragma unroll
-                        for (int i = 0; i < kBlockN; i += 4) {
-                            const float2 xa = __ffma2_rn(
-                                make_float2(__uint_as_float(sreg[i]), __uint_as_float(sreg[i + 1])), scale2, zero2);
-                            const float2 xb = __ffma2_rn(
-                                make_float2(__uint_as_float(sreg[i + 2]), __uint_as_float(sreg[i + 3])), scale2, zero2);
-                            x[i / 2] = xa;
-                            x[i / 2 + 1] = xb;
-                            mt0 = max3(mt0, xa.x, xb.x);
-                            mt1 = max3(mt1, xa.y, xb.y);
-                        }
+                        scale_only();
                     } else {
                         uint32_t vis[4];
 #pragma unroll
@@ -1042,7 +1057,10 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                             mt1 = max3(mt1, xa.y, xb.y);
                         }
                     }
+                } else if (plain_mask) {
+                    scale_only();
                 } else {
+                if constexpr (LIST) mstep += dummy ? 0 : 1;
 #pragma unroll
                 for (int pn = 0; pn < 2; ++pn) {
 #pragma unroll
@@ -1596,7 +1614,7 @@ __device__ unsigned int g_skip_ticket = 0;
 __global__ void __launch_bounds__(256)
 fa_mask_classify_kernel(const uint16_t* __restrict__ mask, long long bs, long long rs, int Sq, int Sk,
                         uint32_t neg_inf2, unsigned char* __restrict__ flags, int* hint,
-                        unsigned int* unit_counter, int region_rows) {
+                        unsigned int* unit_counter, int region_rows, int find_plain) {
     const int nt = blockIdx.x, mp = blockIdx.y, b = blockIdx.z;
     pdl_launch_dependents();
     pdl_wait_prior_grid();                          // the kernel before may have written the mask
@@ -1606,7 +1624,7 @@ fa_mask_classify_kernel(const uint16_t* __restrict__ mask, long long bs, long lo
     const int rsub = threadIdx.x >> 4;              // 16 rows per pass
     const int col = nt * kBlockN + vec * 8;
     const uint16_t neg_inf = static_cast<uint16_t>(neg_inf2 & 0xffffu);
-    int visible = 0;
+    int visible = 0, nonzero = 0;
     // A region is `region_rows` = 256 rows (a query pair) or 128 rows (a tile shared by a pair of
     // heads) of one key block.  Passes of 16 rows in two rounds: 4 passes, a block-wide vote (a
     // region with anything visible usually ends here), then the others with all their loads in
@@ -1627,7 +1645,9 @@ fa_mask_classify_kernel(const uint16_t* __restrict__ mask, long long bs, long lo
             if (!in[u]) continue;
             if (col + 8 <= Sk) {
                 visible |= (v[u].x != neg_inf2) | (v[u].y != neg_inf2) | (v[u].z != neg_inf2) | (v[u].w != neg_inf2);
+                nonzero |= ((v[u].x | v[u].y | v[u].z | v[u].w) & 0x7fff7fffu) != 0u;      // (-0 is zero)
             } else {
+                nonzero = 1;                          // a ragged block needs its tail hidden: never plain
                 const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
@@ -1638,20 +1658,25 @@ fa_mask_classify_kernel(const uint16_t* __restrict__ mask, long long bs, long lo
         }
     };
     scan(std::integral_constant<int, 4>{}, 0);
+    if ((nt + 1) * kBlockN > Sk || !find_plain) nonzero = 1;
     visible = __syncthreads_or(visible) ? 1 : 0;
-    if (!visible) {
+    nonzero = __syncthreads_or(nonzero) ? 1 : 0;
+    if (!visible || !nonzero) {            // all hidden or all zero so far: the rest decides
         if (region_rows > kBlockM) scan(std::integral_constant<int, 12>{}, 4);
         else scan(std::integral_constant<int, 4>{}, 4);
         visible = __syncthreads_or(visible) ? 1 : 0;
+        nonzero = __syncthreads_or(nonzero) ? 1 : 0;
     }
+    const bool mixed = visible && nonzero;
     if (threadIdx.x == 0) {
-        flags[(static_cast<long long>(b) * gridDim.y + mp) * gridDim.x + nt] = visible ? 1 : 0;
+        flags[(static_cast<long long>(b) * gridDim.y + mp) * gridDim.x + nt] =
+            !visible ? 0 : nonzero ? kFlagMixed : kFlagPlain;
         // Tell the host whether this mask has regions worth skipping: the CTAs tally on the
         // device and the last one to finish writes the total, once, to a word of mapped
         // pinned host memory that the host reads on a later call without synchronising.
         // (Only a heuristic input: overlapping launches may blur the tally, never a result.)
         if (hint != nullptr) {
-            if (!visible) atomicAdd(&g_skip_count, 1u);
+            if (!mixed) atomicAdd(&g_skip_count, 1u);
             __threadfence();
             const unsigned int total = gridDim.x * gridDim.y * gridDim.z;
             if (atomicAdd(&g_skip_ticket, 1u) == total - 1) {
@@ -2390,6 +2415,9 @@ static int* g_flag_tally = nullptr;           // kMaxDevices * kFlagSlots ints, 
 static void* g_flag_cache_addr[kMaxDevices] = {};
 static std::mutex g_flag_mutex;
 
+// Telling a block whose mask is zero throughout from a mixed one means reading all of it, which the
+// heads that then do without its tile have to earn.
+constexpr int kPlainMinHeads = 8;
 enum : int { kFlagsOff = 0, kFlagsFill = 1, kFlagsHit = 2, kFlagsHitNothing = 3 };
 // Looks the key up.  kFlagsFill: *flags is a slot the caller must fill with the pre-pass on
 // `stream` (tallying into *tally) and then seal with flag_cache_filled(); kFlagsHit: *flags holds
@@ -2594,7 +2622,8 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
         const dim3 cgrid(plan.kv_blocks, regions, a->batch);
         const uint32_t ninf = a->dtype == FA_SM100_BF16 ? 0xFF80FF80u : 0xFC00FC00u;
         if (!launch_chained(fa_mask_classify_kernel, cgrid, 256, 0, stream, mask_ptr, mask_bs, mask_rs, a->seqlen_q,
-                            a->seqlen_k, ninf, flags, hint_counter, unit_counter, region_rows))
+                            a->seqlen_k, ninf, flags, hint_counter, unit_counter, region_rows,
+                            a->heads >= kPlainMinHeads ? 1 : 0))
             return cuda_failed(__LINE__);
         kp.block_flags = flags;
         kp.unit_counter = unit_counter;

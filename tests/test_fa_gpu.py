@@ -880,3 +880,26 @@ def test_rule_attention_over_long_keys_is_split(dtype, case):
         assert (got_lse[fin] - want_lse[fin]).abs().max().item() <= 1e-4
     check_against_oracle(got, q, k, v, m[..., :sk].contiguous(), f"rule_split{case}")
     assert _cabi.device_status(0, clear=True) == 0
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("case", [
+    # b, h, hk, sq, sk, d: eight heads and more, so that the pre-pass also looks for all-zero blocks
+    (1, 8, 8, 700, 1100, 128), (2, 8, 2, 512, 1024, 64), (1, 16, 4, 40, 1411, 128),
+])
+def test_blocks_without_any_mask_value_need_no_mask_tile(dtype, case):
+    """Key blocks whose mask is zero throughout are computed without their mask tile, in between
+    blocks that need theirs: bit-identical to the run that loads every tile."""
+    b, h, hk, sq, sk, d = case
+    q, k, v, m = _cuda(*make_case(b, h, hk, sq, sk, d, dtype, "zero", seed=71))
+    m[..., 128:256] = float("-inf")                       # a hidden block
+    m[:, :, :, 256:384] = -0.0                            # zero with the sign bit set
+    m[:, :, sq - 1, 511] = 0.5                            # one value in a region's last row and column
+    m[:, :, 0, 512] = float("-inf")                       # ... in its first row and column
+    m[:, :, sq // 2, 700] = -2.0
+    m = m.contiguous()
+    out, lse, plan = run_cabi(q, k, v, m, want_lse=True, num_splits=1, no_unit_cut=1)
+    full, full_lse, _ = run_cabi(q, k, v, m, want_lse=True, num_splits=1, no_unit_cut=1, no_tile_skip=1)
+    assert plan.tile_skip == 1
+    assert torch.equal(out, full) and torch.equal(lse, full_lse)
+    check_against_oracle(out, q, k, v, m, f"plain{case}")
