@@ -903,3 +903,70 @@ def test_blocks_without_any_mask_value_need_no_mask_tile(dtype, case):
     assert plan.tile_skip == 1
     assert torch.equal(out, full) and torch.equal(lse, full_lse)
     check_against_oracle(out, q, k, v, m, f"plain{case}")
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_chained_launches_behind_copies_memsets_and_joined_streams(captured):
+    """Every kernel is launched chained to the work ahead of it in the stream, whatever that is - a
+    copy, a memset, another stream that was joined, another of the library's kernels that writes its
+    operands - eagerly and captured into a graph: always the same bits as with the device idle."""
+    from custom_ops_b200 import ops
+    from custom_ops_b200.masks import rule_attention
+    q, k, v, m = _cuda(*make_case(2, 8, 2, 300, 900, 64, torch.bfloat16, "drop10", seed=73))
+    first = ops.mha_fwd_with_mask(q, k, v, m)
+    torch.cuda.synchronize()
+    want = ops.mha_fwd_with_mask(first, k, v, m)
+    torch.cuda.synchronize()
+    want_rule = rule_attention(want, k, v, causal=True)
+    torch.cuda.synchronize()
+    qb, kb, vb, mid = (torch.empty_like(t) for t in (q, k, v, q))
+    side = torch.cuda.Stream()
+
+    def step():
+        main = torch.cuda.current_stream()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            kb.copy_(k)
+            vb.zero_()
+            vb.add_(v)
+        qb.copy_(q)                                      # a copy directly ahead
+        main.wait_stream(side)                           # ... and a join
+        mid.copy_(ops.mha_fwd_with_mask(qb, kb, vb, m))
+        out = ops.mha_fwd_with_mask(mid, kb, vb, m)
+        return out, rule_attention(out, kb, vb, causal=True)
+
+    if captured:
+        warm = torch.cuda.Stream()
+        warm.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(warm):
+            step()
+        torch.cuda.current_stream().wait_stream(warm)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out, rule = step()
+    for _ in range(3):
+        for t in (qb, kb, vb, mid):
+            t.fill_(float("nan"))
+        if captured:
+            graph.replay()
+        else:
+            out, rule = step()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and torch.equal(rule, want_rule)
+
+
+def test_static_scratch_takes_packed_heads_whose_split_would_not_fit():
+    """64 packed heads over 49001 keys: the partials of the split beside the re-pitched mask are more
+    than the built-in scratch, so that entry point makes one pass and still accepts the call."""
+    q, k, v, m = _cuda(*make_case(1, 64, 8, 64, 49001, 128, torch.bfloat16, "drop10", seed=79))
+    want, _, plan = run_cabi(q, k, v, m, num_splits=1, no_unit_cut=1)
+    _, _, auto = run_cabi(q, k, v, m)
+    assert auto.workspace_bytes > 24 << 20 >= plan.workspace_bytes
+    out = torch.empty_like(q)
+    args = _cabi.make_args(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), mask=m.data_ptr(), out=out.data_ptr(), batch=1,
+                           heads=64, heads_k=8, seqlen_q=64, seqlen_k=49001, head_dim=128, dtype=_cabi.BF16,
+                           mask_seqlen_q=64, mask_seqlen_k=49001, mask_batch_stride=m.stride(0),
+                           mask_row_stride=m.stride(2))
+    _cabi.forward_static_scratch(args, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
