@@ -1458,8 +1458,7 @@ __device__ __forceinline__ void st_release_sys_u32(unsigned int* p, unsigned int
 
 template <int D>
 __global__ void __launch_bounds__(256)
-fa_mask_combine_kernel(const float* __restrict__ o_parts, const float* __restrict__ lse_parts,
-                       void* __restrict__ out, float* __restrict__ lse_out, int num_parts,
+fa_mask_combine_kernel(const float* o_parts, const float* lse_parts, void* out, float* lse_out, int num_parts,
                        long long rows, int is_bf16, int out_fp32, long long o_part_stride,
                        long long lse_part_stride, const PeerExchange px) {
     constexpr int VEC = D / 32;
@@ -1507,8 +1506,8 @@ fa_mask_combine_kernel(const float* __restrict__ o_parts, const float* __restric
         const int s = c * 32 + lane;
         lse_r[c] = -INFINITY;
         if (s < num_parts)
-            lse_r[c] = peers ? ld_cg_f32(px.parts[s] + px.part_offset + rows * D + row)
-                             : lse_parts[static_cast<long long>(s) * lse_part_stride + row];
+            lse_r[c] = ld_cg_f32(peers ? px.parts[s] + px.part_offset + rows * D + row
+                                       : lse_parts + static_cast<long long>(s) * lse_part_stride + row);
         mx = fmaxf(mx, lse_r[c]);
     }
 #pragma unroll
@@ -1541,27 +1540,18 @@ fa_mask_combine_kernel(const float* __restrict__ o_parts, const float* __restric
                 w[u] = __shfl_sync(0xffffffffu, w_r[c], s2 + u);       // same in every lane
                 f[u] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (part < num_parts && w[u] != 0.f) {
-                    // (another GPU's memory is read past the L1: the same addresses carry new
-                    // data every other call)
+                    // (past the L1: the same addresses carry new data every call, another GPU's memory
+                    // every other one, and the kernel before writes them while this one is resident)
                     const float* src = (peers ? px.parts[part] + px.part_offset
                                               : o_parts + static_cast<long long>(part) * o_part_stride) +
                                        row * D + lane * VEC;
                     if constexpr (VEC == 4) {
-                        if (peers) {
-                            const uint4 g = ld_cg_v4(src);
-                            f[u] = make_float4(__uint_as_float(g.x), __uint_as_float(g.y), __uint_as_float(g.z),
-                                               __uint_as_float(g.w));
-                        } else {
-                            f[u] = __ldg(reinterpret_cast<const float4*>(src));
-                        }
+                        const uint4 g = ld_cg_v4(src);
+                        f[u] = make_float4(__uint_as_float(g.x), __uint_as_float(g.y), __uint_as_float(g.z),
+                                           __uint_as_float(g.w));
                     } else {
-                        if (peers) {
-                            f[u].x = ld_cg_f32(src);
-                            f[u].y = ld_cg_f32(src + 1);
-                        } else {
-                            const float2 g = __ldg(reinterpret_cast<const float2*>(src));
-                            f[u].x = g.x; f[u].y = g.y;
-                        }
+                        const float2 g = ld_cg_v2(src);
+                        f[u].x = g.x; f[u].y = g.y;
                     }
                 } else {
                     w[u] = 0.f;
@@ -1617,8 +1607,8 @@ __device__ unsigned int g_skip_count = 0;
 __device__ unsigned int g_skip_ticket = 0;
 
 __global__ void __launch_bounds__(256)
-fa_mask_classify_kernel(const uint16_t* __restrict__ mask, long long bs, long long rs, int Sq, int Sk,
-                        uint32_t neg_inf2, unsigned char* __restrict__ flags, int* hint,
+fa_mask_classify_kernel(const uint16_t* mask, long long bs, long long rs, int Sq, int Sk,
+                        uint32_t neg_inf2, unsigned char* flags, int* hint,
                         unsigned int* unit_counter, int region_rows, int find_plain) {
     const int nt = blockIdx.x, mp = blockIdx.y, b = blockIdx.z;
     pdl_wait_prior_grid();                          // the kernel before may have written the mask
@@ -1643,7 +1633,7 @@ fa_mask_classify_kernel(const uint16_t* __restrict__ mask, long long bs, long lo
             const int row = mp * region_rows + (pass0 + u) * 16 + rsub;
             in[u] = row < Sq && col < Sk;
             v[u] = make_uint4(neg_inf2, neg_inf2, neg_inf2, neg_inf2);
-            if (in[u]) v[u] = __ldg(reinterpret_cast<const uint4*>(mask + b * bs + row * rs + col));
+            if (in[u]) v[u] = ld_cg_v4(mask + b * bs + row * rs + col);
         }
 #pragma unroll
         for (int u = 0; u < kPasses; ++u) {
@@ -1700,7 +1690,7 @@ fa_mask_classify_kernel(const uint16_t* __restrict__ mask, long long bs, long lo
 // get 0; the attention kernel masks columns >= Sk itself.
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-fa_mask_repitch_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int Sq, int Sk,
+fa_mask_repitch_kernel(const uint16_t* src, uint16_t* dst, int Sq, int Sk,
                        int pitch, long long src_bs, long long src_rs) {
     // in this order: whatever runs behind the announcement finds the kernels before this one finished,
     // so the attention kernel may load q, k and v under this kernel (KParams.operands_ready)
@@ -1722,11 +1712,11 @@ fa_mask_repitch_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ 
         uint4 out = make_uint4(0u, 0u, 0u, 0u);
         if (c < Sk) {
             const int valid = min(8, Sk - c);                         // elements wanted from the source
-            const uint4 lo = __ldg(s16 + (c >> 3));
+            const uint4 lo = ld_v4(s16 + (c >> 3));
             // the second vector only when a wanted byte lies in it (never reads past the vector
             // that holds the row's last element)
             uint4 hi = make_uint4(0u, 0u, 0u, 0u);
-            if (mis + 2u * valid > 16u) hi = __ldg(s16 + (c >> 3) + 1);
+            if (mis + 2u * valid > 16u) hi = ld_v4(s16 + (c >> 3) + 1);
             const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
             uint32_t o[4];
             switch (word_off) {                                       // uniform over the CTA
@@ -1771,8 +1761,8 @@ __global__ void fa_zero_counter_kernel(unsigned int* counter) {
 // Mask from rules (padding / causal / sliding window): one 16-byte vector per thread.
 // ---------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-fa_mask_build_kernel(uint16_t* __restrict__ mask, int Sq, int Sk, int pitch, uint32_t neg_inf16, int causal,
-                     int window, const int* __restrict__ valid_lens) {
+fa_mask_build_kernel(uint16_t* mask, int Sq, int Sk, int pitch, uint32_t neg_inf16, int causal,
+                     int window, const int* valid_lens) {
     pdl_launch_dependents();
     pdl_wait_prior_grid();
     const long long r = blockIdx.x;                   // b * Sq + i
@@ -2127,7 +2117,8 @@ static int encode_map(CUtensorMap* tm, const void* ptr, int dtype, int planes, i
 // as soon as all of that kernel's CTAs have started and SMs are free, run what needs no memory of
 // the caller's, and wait (griddepcontrol.wait) for the kernel before to finish and its writes to be
 // visible.  Behind a kernel that does not announce its dependents the wait ends with that kernel.
-// Every kernel here executes the wait, so "the kernel before has finished" covers all before it.
+// Every kernel here executes the wait, so "the kernel before has finished" covers all before it.  None
+// takes a __restrict__ pointer or reads through __ldg: what it reads may be written while it is resident.
 // Back to back calls, before and after: 1.3 MB of operands 12.3 -> 8.2 us, a decode step over 8 x 4096
 // keys 26.6 -> 22.1 us, Split-KV over 32768 keys 73.7 -> 69.8 us.
 template <typename Kern, typename... Args>

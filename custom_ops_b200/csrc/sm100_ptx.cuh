@@ -252,12 +252,28 @@ __device__ __forceinline__ void stg256(void* gptr, const uint32_t* r) {
                  : "memory");
 }
 
-// Loads that bypass the L1 (data another CTA of the same launch wrote), and the acquire /
-// release pair that orders them.
+// Loads of data that another CTA of the same launch, or a kernel that this launch is chained to, wrote
+// while this kernel was already resident.  Never the read-only path (ld.global.nc: __ldg, or any load
+// through a const __restrict__ kernel argument): that one is for memory nobody writes during the kernel's
+// whole lifetime, which begins before griddepcontrol.wait, and the compiler may move it ahead of the wait.
+// ld_cg_* bypass the L1; ld_v4 does not, for vectors that neighbouring threads read too.
+__device__ __forceinline__ uint4 ld_v4(const void* gptr) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(gptr) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ uint4 ld_cg_v4(const void* gptr) {
     uint4 v;
     asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(gptr) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ float2 ld_cg_v2(const void* gptr) {
+    float2 v;
+    asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(gptr) : "memory");
     return v;
 }
 
@@ -267,6 +283,7 @@ __device__ __forceinline__ float ld_cg_f32(const float* gptr) {
     return v;
 }
 
+// ... and the acquire / release pair that orders them.
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* gptr) {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(gptr) : "memory");

@@ -308,3 +308,13 @@ def test_plan_unit_cut_rule():
     assert _plan(batch=1, heads=sm // 2, heads_k=sm // 2, seqlen_q=256, seqlen_k=128 * 16,
                  no_unit_cut=1).grid_x == sm // 2
 
+
+def test_chained_kernels_read_nothing_through_the_read_only_path():
+    """Every kernel is launched chained to the one before it and is resident while that one still
+    writes.  Read-only loads (``__ldg``, or loads through a ``const __restrict__`` argument) are for
+    memory that nobody writes during the kernel's lifetime, and the compiler may move them ahead of the
+    wait for the kernel before; no such load may come back."""
+    csrc = os.path.join(ROOT, "custom_ops_b200", "csrc")
+    for name in ("fa_mask_fwd_sm100.cu", "sm100_ptx.cuh"):
+        code = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        assert not re.findall(r"__ldg\b|__restrict__|ld\.global\.nc", code), name
