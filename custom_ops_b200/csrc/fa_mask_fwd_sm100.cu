@@ -1662,7 +1662,6 @@ fa_mask_classify_kernel(const uint16_t* mask, long long bs, long long rs, int Sq
         visible = __syncthreads_or(visible) ? 1 : 0;
         nonzero = __syncthreads_or(nonzero) ? 1 : 0;
     }
-    const bool mixed = visible && nonzero;
     if (threadIdx.x == 0) {
         flags[(static_cast<long long>(b) * gridDim.y + mp) * gridDim.x + nt] =
             !visible ? 0 : nonzero ? kFlagMixed : kFlagPlain;
@@ -1670,8 +1669,11 @@ fa_mask_classify_kernel(const uint16_t* mask, long long bs, long long rs, int Sq
         // device and the last one to finish writes the total, once, to a word of mapped
         // pinned host memory that the host reads on a later call without synchronising.
         // (Only a heuristic input: overlapping launches may blur the tally, never a result.)
+        // Hidden regions only: what all-zero ones save does not pay for the pre-pass and for units
+        // that are not cut.  Counting them too kept masks with nothing hidden on this path: zeros over
+        // 4 x 16 x 2048 x 2048 150.8 us against 147.1, over 8 heads x 512 x 2048 41.7 against 31.1.
         if (hint != nullptr) {
-            if (!mixed) atomicAdd(&g_skip_count, 1u);
+            if (!visible) atomicAdd(&g_skip_count, 1u);
             __threadfence();
             const unsigned int total = gridDim.x * gridDim.y * gridDim.z;
             if (atomicAdd(&g_skip_ticket, 1u) == total - 1) {

@@ -905,6 +905,24 @@ def test_blocks_without_any_mask_value_need_no_mask_tile(dtype, case):
     check_against_oracle(out, q, k, v, m, f"plain{case}")
 
 
+@pytest.mark.parametrize("version", [0, 3])
+@pytest.mark.parametrize("kind", ["zero", "bias"])
+def test_masks_with_zero_blocks_but_none_hidden_leave_the_pre_pass(kind, version):
+    """All-zero blocks alone do not pay for the pre-pass, whose launches never cut units: a mask that
+    hides nothing ends up on the plain kernel, cut in pieces, also when some or all of its blocks are zero."""
+    q, k, v, m = _cuda(*make_case(1, 8, 8, 512, 2048, 128, torch.bfloat16, "zero" if kind == "zero" else "random", seed=83))
+    m[:, :, :256, :128] = 0.0
+    want, _, plan = run_cabi(q, k, v, m, no_tile_skip=1)
+    assert plan.unit_cut >= 2
+    for _ in range(3):                         # (run_cabi synchronises: the pre-pass has reported)
+        run_cabi(q, k, v, m, mask_version=version)
+    n0 = _cabi.launch_count()
+    out, _, plan = run_cabi(q, k, v, m, mask_version=version)
+    assert plan.tile_skip == 1 and plan.unit_cut >= 2
+    assert _cabi.launch_count() - n0 == 1
+    assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("captured", [False, True])
 def test_chained_launches_behind_copies_memsets_and_joined_streams(captured):
     """Every kernel is launched chained to the work ahead of it in the stream, whatever that is - a
