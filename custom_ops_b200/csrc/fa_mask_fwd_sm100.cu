@@ -153,10 +153,10 @@ struct KParams {
     // (the launcher zeroes it on the stream before the kernel).
     int rule_causal, rule_window;
     const int* valid_lens;
-    // PACK kernels, for few rows or few units.  The query heads of one KV group are consecutive rows
-    // of one "head" (q, out, lse and the partials have that layout as they are), so H = Hk here and
-    // Sq = group size * pack_sq; row r of it is query r % pack_sq, and every tile reads the same pack_sq
-    // mask rows.  A rule launch whose units are cut or split is one of these too, packed or not
+    // PACK kernels, for few rows or few units.  n query heads of one KV group (all of them, or a divisor
+    // of their number) are consecutive rows of one "head" (q, out, lse and the partials have that layout
+    // as they are): H counts those heads, Sq = n * pack_sq, row r is query r % pack_sq, and every tile reads
+    // the same pack_sq mask rows.  A rule launch whose units are cut or split is one of these too, packed or not
     // (pack_sq = Sq): what a cut under a rule needs stays out of the kernel for many units, which it
     // made 3 % slower (a causal window over 2048 keys: 65.9 us against 63.8).
     int pack_sq;
@@ -1917,7 +1917,7 @@ static unsigned long long next_cut_tag() {
 }
 
 // The problem as the kernel sees it.  With few query rows and grouped heads, the rows of all heads
-// of a KV group are packed into one "head" (KParams.pack_sq): a decode step then reads every key
+// of a KV group, or of a part of it, are packed into one "head" (KParams.pack_sq): a decode step then reads every key
 // block once per group instead of once per pair of heads, and the heads left are few enough to split
 // the keys over the GPU (one row, 16 heads in groups of four, 8 x 4096 keys: 74 -> 27 us).  From 65
 // rows on a group of two fills two tiles either way, and the head pairs keep their finer tile skipping.
@@ -1926,11 +1926,18 @@ struct Shape {
     int H, Hk, Sq;
     int pack;          // query rows per head, 0: heads are not packed
 };
+// A split that the caller asks for packs only as many heads as fill one tile (the largest divisor of
+// the group that does): every split then needs what it needs unpacked, half a partial, since a CTA
+// takes two splits of one tile and merges them itself.
 static Shape kernel_shape(const FaMaskFwdArgs* a) {
-    const int group = a->heads / a->heads_k;
-    if (group > 1 && a->seqlen_q > 0 && a->seqlen_q <= kPackMaxRows && (a->disable & FA_SM100_NO_HEAD_PAIRS) == 0)
-        return {a->heads_k, a->heads_k, group * a->seqlen_q, a->seqlen_q};
-    return {a->heads, a->heads_k, a->seqlen_q, 0};
+    const int group = a->heads / a->heads_k, sq = a->seqlen_q;
+    int heads = 1;                                             // heads that share a set of tiles
+    if (sq > 0 && sq <= kPackMaxRows && (a->disable & FA_SM100_NO_HEAD_PAIRS) == 0) {
+        heads = group;
+        if (a->num_splits > 1 && a->seqlen_k > kBlockN)
+            while (heads > 1 && (group % heads != 0 || heads * sq > kBlockM)) --heads;
+    }
+    return {a->heads / heads, a->heads_k, heads * sq, heads > 1 ? sq : 0};
 }
 
 // A mask given by rules instead of a tensor (see KParams): what fa_mask_fwd_sm100_rule passes on.
@@ -2733,11 +2740,12 @@ static int forward_static_scratch(const FaMaskFwdArgs* args, cudaStream_t stream
     FaMaskFwdPlan plan;
     int rc = make_plan(args, &plan);
     if (rc != FA_SM100_OK) return rc;
-    // Packed heads are split where the same call unpacked would not be, or less: where those partials
-    // do not fit, one pass of whole units needs no more scratch than any unpacked plan.
+    // Packed heads are split or cut where the same call unpacked would not be, or less: where those partials
+    // do not fit, one pass of whole units needs no more scratch than any unpacked plan.  (A split that the
+    // caller asks for needs what it needs unpacked, see kernel_shape.)
     FaMaskFwdArgs one_pass = *args;
     const FaMaskFwdArgs* a = args;
-    if (plan.workspace_bytes > FA_SM100_STATIC_SCRATCH_BYTES && args->num_splits == 0 && kernel_shape(args).pack) {
+    if (plan.workspace_bytes > FA_SM100_STATIC_SCRATCH_BYTES && args->num_splits <= 1 && kernel_shape(args).pack) {
         one_pass.num_splits = 1;
         one_pass.disable |= FA_SM100_NO_UNIT_CUT;
         a = &one_pass;

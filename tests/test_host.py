@@ -318,3 +318,30 @@ def test_chained_kernels_read_nothing_through_the_read_only_path():
     for name in ("fa_mask_fwd_sm100.cu", "sm100_ptx.cuh"):
         code = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
         assert not re.findall(r"__ldg\b|__restrict__|ld\.global\.nc", code), name
+
+
+@pytest.mark.parametrize("sq", [1, 16, 17, 33, 64])
+@pytest.mark.parametrize("heads_k", [1, 2, 4, 8])
+@pytest.mark.parametrize("num_splits", [2, 3, 32, 128])
+def test_packed_heads_need_no_more_scratch_for_a_given_split(sq, heads_k, num_splits):
+    """With few query rows grouped heads share query tiles.  A split that the caller asks for then needs
+    the scratch that it needs with the heads apart, so nothing that fits the built-in array is refused."""
+    for group in (2, 3, 4, 6, 7, 8, 12):
+        shape = dict(batch=2, heads=heads_k * group, heads_k=heads_k, seqlen_q=sq, seqlen_k=4096, num_splits=num_splits)
+        p, apart = _plan(**shape), _plan(no_head_pairs=1, **shape)
+        assert p.num_splits == apart.num_splits and p.dual_split == apart.dual_split == 1
+        assert p.workspace_bytes == apart.workspace_bytes
+    assert _plan(batch=2, heads=16, heads_k=2, seqlen_q=64, seqlen_k=4096,
+                 num_splits=32).workspace_bytes <= _cabi.STATIC_SCRATCH_BYTES
+
+
+@pytest.mark.parametrize("num_splits", [0, 1])
+def test_built_in_scratch_takes_packed_heads_beside_a_re_pitched_mask(num_splits):
+    """Packed heads may be split or cut where the heads apart would not be.  Where those partials do not
+    fit the built-in scratch beside the mask's copy, that entry point makes one pass: it does not refuse."""
+    shape = dict(batch=3, heads=64, heads_k=4, seqlen_q=50, seqlen_k=49001, head_dim=128, dtype=_cabi.BF16,
+                 num_splits=num_splits)
+    assert _plan(**shape).workspace_bytes > _cabi.STATIC_SCRATCH_BYTES
+    lib = _cabi.load()
+    refused = lib.fa_mask_fwd_sm100_static_scratch(ctypes.byref(_cabi.make_args(**shape)), None) == -6
+    assert not refused                       # (no pointers, or no GPU here: another error)
