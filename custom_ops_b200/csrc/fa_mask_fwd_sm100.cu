@@ -1922,20 +1922,38 @@ static unsigned long long next_cut_tag() {
 // the keys over the GPU (one row, 16 heads in groups of four, 8 x 4096 keys: 74 -> 27 us).  From 65
 // rows on a group of two fills two tiles either way, and the head pairs keep their finer tile skipping.
 constexpr int kPackMaxRows = 64;
+// Key blocks from which a launch with too few units is split over the keys (make_plan).
+constexpr int kOneTileSplitBlocks = 8, kTilesSplitBlocks = 24;
 struct Shape {
     int H, Hk, Sq;
     int pack;          // query rows per head, 0: heads are not packed
 };
-// A split that the caller asks for packs only as many heads as fill one tile (the largest divisor of
-// the group that does): every split then needs what it needs unpacked, half a partial, since a CTA
-// takes two splits of one tile and merges them itself.
-static Shape kernel_shape(const FaMaskFwdArgs* a) {
+// Only as many heads as fill one tile (the largest divisor of the group that does, possibly one) are
+// packed for
+// - a split that the caller asks for: a CTA then takes two splits of one tile and merges them itself, so
+//   the split needs the scratch that it needs unpacked;
+// - 8 to 23 key blocks and at most half as many heads, counted after packing, as SMs: several tiles are
+//   not split below 24 blocks (see make_plan), one tile is.  64 rows, 32 heads in groups of four, B = 1:
+//   16 blocks 22.8 us (one head per tile, as it was) against 29.8 whole group, 22 blocks 25.0 against 33.5,
+//   11 blocks 26.9 against 26.7; from 24 blocks on, where both are split, the whole group is the faster
+//   one: 24 blocks 22.8 against 20.1, 64 blocks 34.6 against 25.9.  Nor is there anything to gain once
+//   the units fill the GPU: 16 blocks, 12 heads in groups of three, 50 rows, B = 16: 61.8 against 36.4.
+//   (With such a plan, as built: 16 blocks 19.1, 22 blocks 19.6, 11 blocks 22.2.)
+// - fewer blocks, as few heads, and an odd number of tiles per group: SMs are free, and a tile of its own
+//   in a CTA is faster than two that take turns (50 rows, 12 heads in groups of three, six blocks: 18.6 us against 21.7).
+static Shape kernel_shape(const FaMaskFwdArgs* a, int sm_count, bool rule) {
     const int group = a->heads / a->heads_k, sq = a->seqlen_q;
-    int heads = 1;                                             // heads that share a set of tiles
-    if (sq > 0 && sq <= kPackMaxRows && (a->disable & FA_SM100_NO_HEAD_PAIRS) == 0) {
-        heads = group;
-        if (a->num_splits > 1 && a->seqlen_k > kBlockN)
-            while (heads > 1 && (group % heads != 0 || heads * sq > kBlockM)) --heads;
+    if (sq <= 0 || sq > kPackMaxRows || (a->disable & FA_SM100_NO_HEAD_PAIRS) != 0)
+        return {a->heads, a->heads_k, sq, 0};
+    int heads = group;                                         // heads that share a set of tiles
+    if (!rule && a->num_splits != 1 && heads * sq > kBlockM) {
+        int fit = heads;
+        while (fit > 1 && (group % fit != 0 || fit * sq > kBlockM)) --fit;
+        const int nb = ceil_div(a->seqlen_k, kBlockN);
+        const long long one_tile_units = static_cast<long long>(a->batch) * (a->heads / fit);
+        const bool one_tile_cta = nb >= kOneTileSplitBlocks || (group / fit) % 2 != 0;    // (else two heads pair up)
+        if (a->num_splits > 1 ? nb > 1 : nb < kTilesSplitBlocks && one_tile_cta && 2 * one_tile_units <= sm_count)
+            heads = fit;
     }
     return {a->heads / heads, a->heads_k, heads * sq, heads > 1 ? sq : 0};
 }
@@ -1959,7 +1977,7 @@ static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan, const RuleSpec
     query_device(a->device, &dev);
     std::memset(plan, 0, sizeof(*plan));
     const int d = a->head_dim;
-    const Shape ks = kernel_shape(a);
+    const Shape ks = kernel_shape(a, dev->sm_count, rule != nullptr);
     int m_pairs = ceil_div(ks.Sq, 2 * kBlockM);
     const int nb = ceil_div(a->seqlen_k, kBlockN);
     const long long base_ctas = static_cast<long long>(m_pairs) * ks.H * a->batch;
@@ -1986,7 +2004,7 @@ static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan, const RuleSpec
         if (a->num_splits > 0) {
             splits = a->num_splits;
         } else if (base_ctas * 5 < static_cast<long long>(dev->sm_count) * 4 &&
-                   nb >= (one_tile ? 8 : 24)) {
+                   nb >= (one_tile ? kOneTileSplitBlocks : kTilesSplitBlocks)) {
             // Too few CTAs to fill the GPU: cut the key range so that about one CTA
             // lands on every SM, keeping at least four key blocks per CTA.  (With more than
             // one query tile a split costs a partial of 256 rows per CTA and a merge kernel
@@ -2535,7 +2553,6 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     FaMaskFwdPlan plan;
     int rc = make_plan(a, &plan, rule);
     if (rc != FA_SM100_OK) return rc;
-    const Shape ks = kernel_shape(a);
     const long long rows = static_cast<long long>(a->batch) * a->heads * a->seqlen_q;
     if (rows == 0) return FA_SM100_OK;
     if (a->q == nullptr || a->out == nullptr) return FA_SM100_ERR_NULL;
@@ -2557,6 +2574,7 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     if (!dev->queried) return FA_SM100_ERR_CUDA;
     if (dev->cc_major != 10) return FA_SM100_ERR_ARCH;
 
+    const Shape ks = kernel_shape(a, plan.sm_count, rule != nullptr);
     const int d = a->head_dim;
     if (a->seqlen_k == 0) {
         // No keys: every row is "fully masked" -> 0, LSE -inf.  A merge over zero parts
@@ -2745,7 +2763,8 @@ static int forward_static_scratch(const FaMaskFwdArgs* args, cudaStream_t stream
     // caller asks for needs what it needs unpacked, see kernel_shape.)
     FaMaskFwdArgs one_pass = *args;
     const FaMaskFwdArgs* a = args;
-    if (plan.workspace_bytes > FA_SM100_STATIC_SCRATCH_BYTES && args->num_splits <= 1 && kernel_shape(args).pack) {
+    if (plan.workspace_bytes > FA_SM100_STATIC_SCRATCH_BYTES && args->num_splits <= 1 &&
+        kernel_shape(args, plan.sm_count, false).pack) {
         one_pass.num_splits = 1;
         one_pass.disable |= FA_SM100_NO_UNIT_CUT;
         a = &one_pass;

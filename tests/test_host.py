@@ -345,3 +345,18 @@ def test_built_in_scratch_takes_packed_heads_beside_a_re_pitched_mask(num_splits
     lib = _cabi.load()
     refused = lib.fa_mask_fwd_sm100_static_scratch(ctypes.byref(_cabi.make_args(**shape)), None) == -6
     assert not refused                       # (no pointers, or no GPU here: another error)
+
+
+@pytest.mark.parametrize("heads,heads_k,sq", [(32, 8, 64), (32, 8, 33), (16, 2, 64), (16, 2, 17), (12, 4, 50), (14, 2, 20),
+                                              (12, 2, 40), (24, 4, 60)])
+def test_packed_heads_of_several_tiles_are_split_like_one(heads, heads_k, sq):
+    """Between 8 and 23 key blocks one query tile is split over the keys and several are not.  Where that
+    is what fills the GPU, packing stops at one tile: never longer key ranges than with the heads apart."""
+    for nb in range(1, 40):
+        for batch in (1, 2, 4, 64):
+            shape = dict(batch=batch, heads=heads, heads_k=heads_k, seqlen_q=sq, seqlen_k=128 * nb)
+            p, apart = _plan(**shape), _plan(no_head_pairs=1, **shape)
+            if 8 <= nb < 24 and apart.dual_split:
+                assert p.dual_split == 1 and p.blocks_per_split <= apart.blocks_per_split
+            if nb >= 24 or batch == 64:                            # whole groups: several tiles
+                assert p.dual_split == 0 and p.q_tiles_per_cta == 2
