@@ -191,6 +191,11 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // the mark a visit list carries on the blocks whose mask is zero throughout.
 enum : unsigned char { kFlagMixed = 1, kFlagPlain = 2 };
 constexpr uint32_t kListPlain = 0x8000u;
+// LIST of the kernel: no visit list, one of the blocks that are not hidden, or one that also marks the
+// all-zero ones.  The last is a kernel of its own: the code that computes a block without its mask tile
+// slows the loop even where it never runs (causal, too few heads for marks: 4 heads x 8192 tokens 173.3 us
+// against 161.8, 16 x 4 x 2048 155.4 against 147.7).
+enum : int { kListNone = 0, kListVisit = 1, kListPlainMarks = 2 };
 enum : int { kPartWhole = 0, kPartTail = 1, kPartHead = 2 };
 
 // Unit board: what the scheduler warp publishes about one unit of work, a (split group,
@@ -281,7 +286,7 @@ struct Ring {
     }
 };
 
-template <int D, bool BF16, bool LIST, bool RULE, bool PACK>
+template <int D, bool BF16, int LIST, bool RULE, bool PACK>
 __global__ void __launch_bounds__(kThreads, 1)
 fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                    const __grid_constant__ CUtensorMap tm_k,
@@ -290,6 +295,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                    const KParams p) {
     using C = Cfg<D>;
     constexpr int NS = C::kStages;
+    constexpr uint32_t kMarks = LIST == kListPlainMarks ? kListPlain : 0u;     // in the entries of a visit list
     constexpr uint32_t TILE = C::kTileBytes;
     constexpr uint32_t SUB = C::kSubBytes;
 
@@ -382,7 +388,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 const unsigned ballot = __ballot_sync(0xffffffffu, need);
                 if (need)
                     sts16(lst + 2 * (count + __popc(ballot & ((1u << lane) - 1u))),
-                          static_cast<uint32_t>(jj) | (fl[jj] == kFlagPlain ? kListPlain : 0u));
+                          static_cast<uint32_t>(jj) | (LIST == kListPlainMarks && fl[jj] == kFlagPlain ? kListPlain : 0u));
                 count += __popc(ballot);
             }
         }
@@ -578,7 +584,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                         if (!dual) {
                             // shared by both slots: K_0, V_0, K_1, V_1, ...
                             for (int j = 0; ok && j < n0; ++j) {
-                                const int blk = LIST ? static_cast<int>(lds16(lst + 2 * j) & ~kListPlain) : begin0 + j;
+                                const int blk = LIST ? static_cast<int>(lds16(lst + 2 * j) & ~kMarks) : begin0 + j;
                                 ok = fill(false, blk) && fill(true, blk);
                             }
                         } else {
@@ -640,7 +646,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                             if (!ok || j >= n_of[t]) continue;
                             if (t == 1 && p.head_pairs) continue;      // slot 1 reads slot 0's panels
                             const int blk = LIST ? static_cast<int>(lds16(lst + 2 * j)) : begin_of[t] + j;
-                            if (LIST && (blk & kListPlain)) continue;      // nothing to add: no tile wanted
+                            if (blk & kMarks) continue;      // nothing to add: no tile wanted
 #pragma unroll
                             for (int hf = 0; hf < 2; ++hf) {
                                 const int i = 2 * t + hf;
@@ -916,7 +922,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
         const float2 scale2 = make_float2(p.scale, p.scale);
 
         int gstep = 0;               // key-block steps of this slot so far, over all units
-        [[maybe_unused]] int mstep = 0;   // LIST: those of them that had a mask tile
+        [[maybe_unused]] int mstep = 0;   // kListPlainMarks: those of them that had a mask tile
         int o_uses = 0;              // units of this slot that waited for their final O
         bool alive = true;
         // The body of a key-block step is some 15 KB of straight-line code, and a launch finds it
@@ -971,9 +977,9 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
             for (; j < n_t; ++j) {
                 const bool dummy = j < 0;
                 const int entry = LIST ? static_cast<int>(lds16(lst + 2 * j)) : begin_t + j;
-                // LIST: a block whose mask is zero throughout has no mask tile in shared memory
-                const bool plain_mask = LIST && !dummy && (entry & kListPlain) != 0;
-                const int col0 = (LIST ? entry & ~static_cast<int>(kListPlain) : entry) * kBlockN;
+                // a block whose mask is zero throughout has no mask tile in shared memory
+                const bool plain_mask = LIST == kListPlainMarks && !dummy && (entry & kListPlain) != 0;
+                const int col0 = (entry & ~static_cast<int>(kMarks)) * kBlockN;
                 const bool tail = !dummy && (col0 + kBlockN) > p.Sk;
                 const uint32_t par = (gstep & 1) ^ (dummy ? 1u : 0u);
 
@@ -984,7 +990,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 // but the wake-up from the score barrier stands between S and the first load.
                 bool ok = true;
                 if (!RULE && !plain_mask) {
-                    const uint32_t m_par = LIST ? (mstep & 1) ^ (dummy ? 1u : 0u) : par;
+                    const uint32_t m_par = LIST == kListPlainMarks ? (mstep & 1) ^ (dummy ? 1u : 0u) : par;
                     ok = mbar_wait(dummy ? bar_scratch : bar_m_full + 8 * (2 * mt), m_par, abort_flag, p.status, kStSoftmaxMask);
                     ok = mbar_wait(dummy ? bar_scratch : bar_m_full + 8 * (2 * mt + 1), m_par, abort_flag, p.status, kStSoftmaxMask) && ok;
                 }
@@ -1063,7 +1069,7 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 } else if (plain_mask) {
                     scale_only();
                 } else {
-                if constexpr (LIST) mstep += dummy ? 0 : 1;
+                if constexpr (LIST == kListPlainMarks) mstep += dummy ? 0 : 1;
 #pragma unroll
                 for (int pn = 0; pn < 2; ++pn) {
 #pragma unroll
@@ -1807,7 +1813,7 @@ struct DeviceInfo {
     unsigned int* status_ptr = nullptr;
     unsigned int* status_host = nullptr;     // pinned, mapped: the kernels' copy of a wait that gave up
     bool status_host_failed = false;
-    bool attr_set[24] = {};                  // per kernel instantiation, see launch_fwd
+    bool attr_set[32] = {};                  // per kernel instantiation, see launch_fwd
     bool queried = false;
 };
 static DeviceInfo g_dev[kMaxDevices];
@@ -2213,12 +2219,12 @@ static int get_maps(const MapKey& key, CUtensorMap* tq, CUtensorMap* tk, CUtenso
     return FA_SM100_OK;
 }
 
-template <int D, bool BF16, bool LIST, bool RULE, bool PACK>
+template <int D, bool BF16, int LIST, bool RULE, bool PACK>
 static int launch_fwd(DeviceInfo* dev, const CUtensorMap& tq, const CUtensorMap& tk,
                       const CUtensorMap& tv, const CUtensorMap& tm, const KParams& kp, dim3 grid,
                       cudaStream_t stream) {
     auto kern = fa_mask_fwd_kernel<D, BF16, LIST, RULE, PACK>;
-    const int slot = (D == 128 ? 0 : 1) + (BF16 ? 0 : 2) + (PACK ? 4 : 0) + (RULE ? 16 : LIST ? 8 : 0);
+    const int slot = (D == 128 ? 0 : 1) + (BF16 ? 0 : 2) + (PACK ? 4 : 0) + 8 * (RULE ? 3 : LIST);
     if (!dev->attr_set[slot]) {
         // The in-kernel register re-balancing is only sound for the register count it was
         // written for; refuse to launch a build that came out different.
@@ -2440,9 +2446,13 @@ static int* g_flag_tally = nullptr;           // kMaxDevices * kFlagSlots ints, 
 static void* g_flag_cache_addr[kMaxDevices] = {};
 static std::mutex g_flag_mutex;
 
-// Telling a block whose mask is zero throughout from a mixed one means reading all of it (a 128 x 128
-// region is 32 KB, some 5 ns of the GPU's bandwidth), which the heads that then do without its tile
-// have to earn (about 1 ns each: 7 % of a step's 2 us, over 148 SMs), so not below eight of them.
+// Telling a block whose mask is zero throughout from a mixed one means reading all of it, which the heads
+// that then do without its tile have to earn.  Causal masks, with marks against without (us):
+//   4 heads  4 x 2048 52.8 / 51.7   16 x 2048 149.2 / 146.0   8192 165.4 / 160.5   d = 64: 8 x 777 35.0 / 36.3
+//   6 heads  4 x 2048 83.4 / 83.1   16 x 2048 191.9 / 189.7   8192 269.3 / 266.4
+//   8 heads  4 x 2048 88.2 / 87.5   16 x 2048 234.2 / 234.2   8192 280.4 / 278.5   d = 64: 8 x 777 51.0 / 54.3
+//                                   fp16 2 x 4096 145.8 / 151.9
+//  16 heads  4 x 2048 128.3 / 128.9                           8192 385 / 400       d = 64: 8 x 777 73.8 / 79.0
 constexpr int kPlainMinHeads = 8;
 enum : int { kFlagsOff = 0, kFlagsFill = 1, kFlagsHit = 2, kFlagsHitNothing = 3 };
 // Looks the key up.  kFlagsFill: *flags is a slot the caller must fill with the pre-pass on
@@ -2540,12 +2550,13 @@ static void flag_cache_read(int device, int slot, cudaStream_t stream) {
 }
 
 template <int D, bool BF16, bool PACK>
-static int launch_variant(bool list, bool rule, DeviceInfo* dev, const CUtensorMap& tq, const CUtensorMap& tk,
+static int launch_variant(int list, bool rule, DeviceInfo* dev, const CUtensorMap& tq, const CUtensorMap& tk,
                           const CUtensorMap& tv, const CUtensorMap& tm, const KParams& kp, dim3 grid,
                           cudaStream_t stream) {
-    if (rule) return launch_fwd<D, BF16, false, true, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
-    if (list) return launch_fwd<D, BF16, true, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
-    return launch_fwd<D, BF16, false, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
+    if (rule) return launch_fwd<D, BF16, kListNone, true, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
+    if (list == kListPlainMarks) return launch_fwd<D, BF16, kListPlainMarks, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
+    if (list == kListVisit) return launch_fwd<D, BF16, kListVisit, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
+    return launch_fwd<D, BF16, kListNone, false, PACK>(dev, tq, tk, tv, tm, kp, grid, stream);
 }
 
 static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_bytes,
@@ -2620,6 +2631,7 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
         mask_rs = pitch;
     }
     int* hint_counter = nullptr;
+    const bool plain_marks = a->heads >= kPlainMinHeads;
     const int region_rows = plan.head_pairs ? kBlockM : 2 * kBlockM;
     const int regions = ceil_div(a->seqlen_q, region_rows);       // (packed heads: one)
     const size_t flag_bytes = static_cast<size_t>(a->batch) * regions * plan.kv_blocks;
@@ -2648,8 +2660,7 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
         const dim3 cgrid(plan.kv_blocks, regions, a->batch);
         const uint32_t ninf = a->dtype == FA_SM100_BF16 ? 0xFF80FF80u : 0xFC00FC00u;
         if (!launch_chained(fa_mask_classify_kernel, cgrid, 256, 0, stream, mask_ptr, mask_bs, mask_rs, a->seqlen_q,
-                            a->seqlen_k, ninf, flags, hint_counter, unit_counter, region_rows,
-                            a->heads >= kPlainMinHeads ? 1 : 0))
+                            a->seqlen_k, ninf, flags, hint_counter, unit_counter, region_rows, plain_marks ? 1 : 0))
             return cuda_failed(__LINE__);
         kp.block_flags = flags;
         kp.unit_counter = unit_counter;
@@ -2721,9 +2732,9 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
 
     const dim3 grid(plan.grid_x, plan.grid_y, plan.grid_z);
     const bool bf16 = a->dtype == FA_SM100_BF16;
-    const bool list = kp.block_flags != nullptr;
+    const int list = kp.block_flags == nullptr ? kListNone : plain_marks ? kListPlainMarks : kListVisit;
     // (a rule launch has no skip list and nothing to re-pitch: fa_mask_fwd_sm100_rule sees to that)
-    if (rule != nullptr && (list || plan.mask_repitched)) return FA_SM100_ERR_SHAPE;
+    if (rule != nullptr && (list != kListNone || plan.mask_repitched)) return FA_SM100_ERR_SHAPE;
     auto launch = [&](auto head_dim, auto is_bf16) {
         constexpr int kD = decltype(head_dim)::value;
         constexpr bool kBf16 = decltype(is_bf16)::value;

@@ -905,6 +905,29 @@ def test_blocks_without_any_mask_value_need_no_mask_tile(dtype, case):
     check_against_oracle(out, q, k, v, m, f"plain{case}")
 
 
+def test_eight_heads_do_without_the_tiles_of_zero_blocks_and_fewer_do_not():
+    """From eight heads on the pre-pass marks all-zero blocks and the kernel wants no mask tile for them:
+    with the mask loads withheld a mask of hidden and all-zero blocks still gives the right result.  With
+    fewer heads a kernel without that code runs, also on flags that a call with eight heads left behind:
+    it waits for the tiles, in vain (the wait is bounded and reported)."""
+    q, k, v, m = _cuda(*make_case(1, 8, 8, 384, 1152, 128, torch.bfloat16, "zero", seed=89))
+    m[..., 512:768] = float("-inf")
+    want, _, _ = run_cabi(q, k, v, m, num_splits=1, no_unit_cut=1, mask_version=11)      # leaves its flags behind
+    stream = torch.cuda.current_stream().cuda_stream
+    for heads, status in ((8, (0,)), (4, (4, 9))):             # (4: the MMA thread saw it first)
+        out = torch.zeros(1, heads, 384, 128, dtype=q.dtype, device="cuda")
+        qh, kh, vh = (t[:, :heads].contiguous() for t in (q, k, v))
+        args = _cabi.make_args(q=qh.data_ptr(), k=kh.data_ptr(), v=vh.data_ptr(), mask=m.data_ptr(), out=out.data_ptr(),
+                               batch=1, heads=heads, heads_k=heads, seqlen_q=384, seqlen_k=1152, head_dim=128,
+                               dtype=_cabi.BF16, num_splits=1, no_unit_cut=1, mask_version=11, test_stall_mask=1)
+        nbytes = _cabi.workspace_bytes(args)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+        _cabi.forward(args, ws.data_ptr(), nbytes, stream)
+        assert _cabi.device_status(0, clear=True) in status
+        if heads == 8:
+            assert torch.equal(out, want)
+
+
 @pytest.mark.parametrize("version", [0, 3])
 @pytest.mark.parametrize("kind", ["zero", "bias"])
 def test_masks_with_zero_blocks_but_none_hidden_leave_the_pre_pass(kind, version):
