@@ -2434,6 +2434,7 @@ struct FlagEntry {
     const void* mask = nullptr;
     long long bs = 0, rs = 0;
     int B = 0, Sq = 0, Sk = 0, dtype = 0, device = 0, region_rows = 0;
+    bool plain_marks = false;      // the pre-pass told all-zero blocks from mixed ones (of use to any reader)
     unsigned long long version = 0;
     bool valid = false;
     cudaStream_t fill_stream = nullptr;
@@ -2460,8 +2461,8 @@ enum : int { kFlagsOff = 0, kFlagsFill = 1, kFlagsHit = 2, kFlagsHitNothing = 3 
 // valid flags (any cross-stream wait is already enqueued); kFlagsHitNothing: the mask is known
 // to have nothing to skip; kFlagsOff: no caching for this call.
 static int flag_cache_lookup(const FaMaskFwdArgs* a, const void* mask, long long bs, long long rs,
-                             int region_rows, size_t flag_bytes, cudaStream_t stream, int* slot_out,
-                             unsigned char** flags, int** tally) {
+                             int region_rows, bool plain_marks, size_t flag_bytes, cudaStream_t stream,
+                             int* slot_out, unsigned char** flags, int** tally) {
     *slot_out = -1;
     if (a->mask_version == 0 || flag_bytes > kFlagSlotBytes) return kFlagsOff;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -2496,7 +2497,7 @@ static int flag_cache_lookup(const FaMaskFwdArgs* a, const void* mask, long long
         FlagEntry& e = entries[i];
         if (e.valid && e.mask == mask && e.bs == bs && e.rs == rs && e.B == a->batch && e.Sq == a->seqlen_q &&
             e.Sk == a->seqlen_k && e.dtype == a->dtype && e.device == a->device &&
-            e.region_rows == region_rows && e.version == a->mask_version) {
+            e.region_rows == region_rows && (e.plain_marks || !plain_marks) && e.version == a->mask_version) {
             // 0: the pre-pass has not reported yet; 1: nothing to skip; > 1: something
             if (*static_cast<volatile int*>(tallies + i) == 1) return kFlagsHitNothing;
             if (e.fill_stream != stream && cudaStreamWaitEvent(stream, e.filled, 0) != cudaSuccess) {
@@ -2525,7 +2526,8 @@ static int flag_cache_lookup(const FaMaskFwdArgs* a, const void* mask, long long
     }
     e.valid = false;                      // sealed by flag_cache_filled()
     e.mask = mask; e.bs = bs; e.rs = rs; e.B = a->batch; e.Sq = a->seqlen_q; e.Sk = a->seqlen_k;
-    e.dtype = a->dtype; e.device = a->device; e.region_rows = region_rows; e.version = a->mask_version;
+    e.dtype = a->dtype; e.device = a->device; e.region_rows = region_rows; e.plain_marks = plain_marks;
+    e.version = a->mask_version;
     e.fill_stream = stream;
     e.read_recorded = false;
     tallies[i] = 0;
@@ -2640,7 +2642,7 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     int flag_slot = -1;
     unsigned char* cached_flags = nullptr;
     const int cache = (plan.tile_skip && adaptive_skip && !plan.mask_repitched)
-        ? flag_cache_lookup(a, mask_ptr, mask_bs, mask_rs, region_rows, flag_bytes, stream, &flag_slot,
+        ? flag_cache_lookup(a, mask_ptr, mask_bs, mask_rs, region_rows, plain_marks, flag_bytes, stream, &flag_slot,
                             &cached_flags, &hint_counter)
         : kFlagsOff;
     const bool run_classify = plan.tile_skip && cache != kFlagsHit && cache != kFlagsHitNothing &&

@@ -928,6 +928,28 @@ def test_eight_heads_do_without_the_tiles_of_zero_blocks_and_fewer_do_not():
             assert torch.equal(out, want)
 
 
+def test_remembered_flags_without_zero_blocks_are_filled_again_for_eight_heads():
+    """Flags that a call with four heads left behind do not tell all-zero blocks from mixed ones: the first
+    call with eight heads under the same version runs the pre-pass once more, the next one does not, and
+    neither wants a mask tile for an all-zero block (the mask loads are withheld)."""
+    q, k, v, m = _cuda(*make_case(1, 8, 8, 384, 1280, 128, torch.bfloat16, "zero", seed=97))
+    m[..., 512:768] = float("-inf")
+    run_cabi(*(t[:, :4].contiguous() for t in (q, k, v)), m, num_splits=1, no_unit_cut=1, mask_version=12)
+    want, _, _ = run_cabi(q, k, v, m, num_splits=1, no_unit_cut=1)
+    args = _cabi.make_args(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), mask=m.data_ptr(), out=q.data_ptr(), batch=1,
+                           heads=8, heads_k=8, seqlen_q=384, seqlen_k=1280, head_dim=128, dtype=_cabi.BF16,
+                           num_splits=1, no_unit_cut=1, mask_version=12, test_stall_mask=1)
+    nbytes = _cabi.workspace_bytes(args)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    for launches in (2, 1):
+        out = torch.zeros_like(q)
+        args.out = out.data_ptr()
+        n0 = _cabi.launch_count()
+        _cabi.forward(args, ws.data_ptr(), nbytes, torch.cuda.current_stream().cuda_stream)
+        assert _cabi.device_status(0, clear=True) == 0
+        assert _cabi.launch_count() - n0 == launches and torch.equal(out, want)
+
+
 @pytest.mark.parametrize("version", [0, 3])
 @pytest.mark.parametrize("kind", ["zero", "bias"])
 def test_masks_with_zero_blocks_but_none_hidden_leave_the_pre_pass(kind, version):
