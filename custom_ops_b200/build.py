@@ -20,6 +20,7 @@ from __future__ import annotations
 import fcntl
 import hashlib
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -84,7 +85,7 @@ def _up_to_date(so: str, fp: str) -> bool:
     if not (os.path.exists(so) and os.path.exists(stamp)):
         return False
     with open(stamp) as f:
-        return f.read().strip() == fp
+        return f.readline().strip() == fp
 
 
 def _run(cmd, what: str, verbose: bool):
@@ -104,7 +105,7 @@ def _locked(so: str):
 
 def build_cabi(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
     """Compile the kernels + C ABI for sm_100a.  Returns the library path."""
-    flags = list(NVCC_FLAGS) + (["-Xptxas", "-v"] if ptxas_info else [])
+    flags = list(NVCC_FLAGS) + ["-Xptxas", "-v"]
     fp = _fingerprint(CABI_SOURCES + CABI_HEADERS, " ".join(flags))
     lock = _locked(CABI_SO)
     try:
@@ -115,12 +116,22 @@ def build_cabi(force: bool = False, verbose: bool = False, ptxas_info: bool = Fa
                  "nvcc (C-ABI library)", verbose)
         if ptxas_info:
             print(r.stderr, file=sys.stderr)
+        spilled = sum(int(n) for n in re.findall(r"(\d+) bytes spill (?:stores|loads)", r.stderr))
+        if spilled:
+            print(f"[custom_ops_b200.build] warning: ptxas spilled registers ({spilled} bytes): the kernels "
+                  "will be slow", file=sys.stderr)
         os.replace(tmp, CABI_SO)
         with open(CABI_SO + ".build_stamp", "w") as f:
-            f.write(fp)
+            f.write(f"{fp}\n{spilled} bytes spilled\n")
         return CABI_SO
     finally:
         lock.close()
+
+
+def spilled_bytes() -> int:
+    """Bytes of register spills, over all kernels, that ptxas reported for the library as it stands."""
+    with open(CABI_SO + ".build_stamp") as f:
+        return int(f.read().split("\n")[1].split()[0])
 
 
 def build_torch_binding(force: bool = False, verbose: bool = False) -> str:

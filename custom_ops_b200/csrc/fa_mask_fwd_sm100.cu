@@ -1034,7 +1034,8 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                     // row's 128 visibility bits are built from the two limits and each score gets
                     // 0 or -inf added (columns beyond Sk lie beyond rule_hi).
                     const int rel_lo = rule_lo - col0, rel_hi = rule_hi - col0;
-                    const bool plain = __all_sync(0xffffffffu, rel_lo < 0 && rel_hi >= kBlockN - 1) && !dummy;
+                    // (the first pass is voted out inside: a test behind the vote made the kernels spill)
+                    const bool plain = __all_sync(0xffffffffu, rel_lo < 0 && rel_hi >= kBlockN - 1 && !dummy);
                     if (plain) {
                         scale_only();
                     } else {
@@ -1265,24 +1266,6 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                         const float* part_o = p.cut_part + (static_cast<long long>(slot) * (2 * kBlockM) + tile_row) * D;
                         const float lse_p = ld_cg_f32(p.cut_part + lse_base + static_cast<long long>(slot) * (2 * kBlockM) +
                                                       tile_row);
-                        // All loads of the partial are issued before the first is used (one at
-                        // a time they cost a trip to the L2 each).  The four lanes of a quad read
-                        // line-sized pieces of their four rows: the inverse of the stores below,
-                        // see quad_transpose.
-                        uint32_t pr[D];
-                        const int q4 = lane & 3;
-#pragma unroll
-                        for (int c = 0; c < D / 32; ++c) {
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const float* src = part_o + (i - q4) * D + c * 32 + q4 * 8;
-                                const uint4 lo = ld_cg_v4(src), hi = ld_cg_v4(src + 4);
-                                pr[c * 32 + 8 * i] = lo.x; pr[c * 32 + 8 * i + 1] = lo.y;
-                                pr[c * 32 + 8 * i + 2] = lo.z; pr[c * 32 + 8 * i + 3] = lo.w;
-                                pr[c * 32 + 8 * i + 4] = hi.x; pr[c * 32 + 8 * i + 5] = hi.y;
-                                pr[c * 32 + 8 * i + 6] = hi.z; pr[c * 32 + 8 * i + 7] = hi.w;
-                            }
-                        }
                         // out = (a_o * O/l + a_p * o_p) / (a_o + a_p),  a = exp(lse - max lse);
                         // the merged, normalised row goes back to tensor memory
                         const float mx = fmaxf(lse_val, lse_p);
@@ -1294,17 +1277,40 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                             w_p = a_p / den;
                             lse_val = mx + __logf(den);
                         }
+                        // 64 columns at a time, all of their loads issued before the first is used (one at
+                        // a time they cost a trip to the L2 each).  The four lanes of a quad read line-sized
+                        // pieces of their four rows: the inverse of the stores below, see quad_transpose.
+                        // (The whole row in flight left no registers for what lives across this block: the
+                        // d = 128 kernels for a mask tensor spilled 12 bytes a thread.)
+                        const int q4 = lane & 3;
+#pragma unroll 1
+                        for (int c0 = 0; c0 < D / 32; c0 += 2) {
+                            uint32_t pr[64];
 #pragma unroll
-                        for (int c = 0; c < D / 32; ++c) {
-                            uint32_t w[32], oc[32];
+                            for (int c = 0; c < 2; ++c) {
 #pragma unroll
-                            for (int i = 0; i < 32; ++i) w[i] = pr[c * 32 + i];
-                            quad_transpose(w, lane);
-                            tmem_ld32(tO + c * 32, oc);
+                                for (int i = 0; i < 4; ++i) {
+                                    const float* src = part_o + (i - q4) * D + (c0 + c) * 32 + q4 * 8;
+                                    const uint4 lo = ld_cg_v4(src), hi = ld_cg_v4(src + 4);
+                                    pr[c * 32 + 8 * i] = lo.x; pr[c * 32 + 8 * i + 1] = lo.y;
+                                    pr[c * 32 + 8 * i + 2] = lo.z; pr[c * 32 + 8 * i + 3] = lo.w;
+                                    pr[c * 32 + 8 * i + 4] = hi.x; pr[c * 32 + 8 * i + 5] = hi.y;
+                                    pr[c * 32 + 8 * i + 6] = hi.z; pr[c * 32 + 8 * i + 7] = hi.w;
+                                }
+                            }
+                            __syncwarp();
 #pragma unroll
-                            for (int i = 0; i < 32; ++i)
-                                oc[i] = __float_as_uint(__uint_as_float(oc[i]) * w_o + __uint_as_float(w[i]) * w_p);
-                            tmem_st32(tO + c * 32, oc);
+                            for (int c = 0; c < 2; ++c) {
+                                uint32_t w[32], oc[32];
+#pragma unroll
+                                for (int i = 0; i < 32; ++i) w[i] = pr[c * 32 + i];
+                                quad_transpose(w, lane);
+                                tmem_ld32(tO + (c0 + c) * 32, oc);
+#pragma unroll
+                                for (int i = 0; i < 32; ++i)
+                                    oc[i] = __float_as_uint(__uint_as_float(oc[i]) * w_o + __uint_as_float(w[i]) * w_p);
+                                tmem_st32(tO + (c0 + c) * 32, oc);
+                            }
                         }
                         tmem_wait_st();
                         // The tag is taken back once the partial has been read (every load above
@@ -1346,9 +1352,8 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                     tmem_wait_st();
                 }
                 // Rolled on purpose: this code runs once per unit, from no instruction cache, so every
-                // line of it costs a miss.  Unrolled over the whole row the epilogue made calls of short
-                // units slower (4 x 2048 x 2048 under a window of 512, as a rule 63.4 us against 60.9, as
-                // a mask tensor 78.1 against 75.7; 16 key blocks per unit: 174.7 against 172.5).
+                // line of it costs a miss; unrolled over the row, sliding windows of 512 over 4 x 2048 x 2048
+                // ran 78.1 us against 75.7.
                 if (wide) {
                     // quad-transposed, line-sized stores (see quad_transpose)
                     if (o32 != nullptr) {

@@ -360,3 +360,11 @@ def test_packed_heads_of_several_tiles_are_split_like_one(heads, heads_k, sq):
                 assert p.dual_split == 1 and p.blocks_per_split <= apart.blocks_per_split
             if nb >= 24 or batch == 64:                            # whole groups: several tiles
                 assert p.dual_split == 0 and p.q_tiles_per_cta == 2
+
+
+def test_no_kernel_spills_registers():
+    """The attention kernel splits the register file between its warps to the last register; a spill
+    puts trips to local memory into loops and epilogues that are bound by latency."""
+    from custom_ops_b200 import build
+    build.build_cabi()
+    assert build.spilled_bytes() == 0
