@@ -273,7 +273,8 @@ RULE_WORKSPACE_BYTES = 16
 
 
 def rule_workspace_bytes(args: FaMaskFwdArgs, window: int) -> int:
-    """Bytes of workspace with which ``forward_rule`` may split the keys over the GPU."""
+    """Bytes of workspace with which ``forward_rule`` may split the keys over the GPU;
+    ``RULE_WORKSPACE_BYTES`` where it does not split (short key ranges, a full GPU, ``no_unit_cut``)."""
     n = ctypes.c_size_t()
     check(load().fa_mask_fwd_sm100_rule_workspace_bytes(ctypes.byref(args), int(window), ctypes.byref(n)))
     return n.value
@@ -282,8 +283,9 @@ def rule_workspace_bytes(args: FaMaskFwdArgs, window: int) -> int:
 def forward_rule(args: FaMaskFwdArgs, causal: int, window: int, valid_lens: int, stream: int,
                  workspace: int = 0, workspace_nbytes: int = 0):
     """The forward for a mask given by rules (causal / sliding window / valid lengths) instead of
-    a tensor; ``valid_lens`` is a device pointer to ``batch`` int32 or 0; ``workspace``:
-    ``RULE_WORKSPACE_BYTES`` of device memory private to the call, or 0."""
+    a tensor; ``valid_lens`` is a device pointer to ``batch`` int32 or 0; ``workspace``: device memory
+    private to the call, ``rule_workspace_bytes()`` of it (long keys may be split), ``RULE_WORKSPACE_BYTES``
+    (one pass) or 0 (one pass, every CTA takes a fixed share of the units)."""
     check(load().fa_mask_fwd_sm100_rule(ctypes.byref(args), int(causal), int(window), valid_lens or None,
                                         workspace or None, workspace_nbytes, stream or None))
 

@@ -2000,7 +2000,8 @@ static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan, const RuleSpec
         const long long most = (span + kBlockN - 1) / kBlockN + 1;
         if (most < nb_unit) nb_unit = static_cast<int>(most);
     }
-    const bool rule_split = rule != nullptr && rule->may_split && nb_unit > kRuleWholeBlocks;
+    const bool rule_split = rule != nullptr && rule->may_split && nb_unit > kRuleWholeBlocks &&
+                            (a->disable & FA_SM100_NO_UNIT_CUT) == 0;
     int splits = 1;
     if (rule != nullptr) {
         // One query tile: an even number of splits, two per CTA, for about one CTA per SM.

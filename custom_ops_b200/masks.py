@@ -11,7 +11,9 @@ ignored by the operator - and no re-pitch copy runs.
 ``rule_attention`` goes one step further: the same rules evaluated inside the attention kernel
 (``fa_mask_fwd_sm100_rule``), so that no mask exists in memory at all - no mask traffic, no
 tile-skip pre-pass (the visible key range of a unit follows from the rule), no mask add on the
-blocks a row sees entirely.  Bit-identical to ``ops.mha_fwd_with_mask(q, k, v, rule_mask(...))``.
+blocks a row sees entirely.  One pass over the keys gives the bits of the operator's single pass on
+``rule_mask(...)``; above 24 blocks of 128 keys, where few rows or heads would leave SMs idle, the keys are
+split and the result differs by the rounding of the merge, unless ``single_pass`` asks for one pass.
 """
 from __future__ import annotations
 
@@ -61,11 +63,15 @@ def rule_mask(batch: int, seqlen_q: int, seqlen_k: int, *, dtype: torch.dtype = 
 
 
 def rule_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal: bool = False, window: int = 0,
-                   valid_lens: Optional[torch.Tensor] = None, return_lse: bool = False):
+                   valid_lens: Optional[torch.Tensor] = None, return_lse: bool = False, single_pass: bool = False):
     """Attention forward of q ``(B, H, Sq, d)`` over k, v ``(B, Hk, Sk, d)`` under the mask that
     ``rule_mask(B, Sq, Sk, causal=..., window=..., valid_lens=...)`` would describe, without
     building it.  Returns ``out`` (and the fp32 ``(B, H, Sq)`` natural-log LSE with ``return_lse``).
-    A row that sees no key gives 0 (LSE -inf)."""
+    A row that sees no key gives 0 (LSE -inf).
+
+    Long keys may be split over the GPU: the result then depends, within one rounding of the output type, on
+    the number of SMs.  ``single_pass`` keeps it to one pass over the keys, whose result does not, at the
+    price of the SMs that this leaves idle."""
     if not (q.is_cuda and k.is_cuda and v.is_cuda):
         raise RuntimeError("rule_attention is only supported on CUDA")
     if q.dtype not in (torch.bfloat16, torch.float16) or k.dtype != q.dtype or v.dtype != q.dtype:
@@ -91,7 +97,7 @@ def rule_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, causal:
     args = _cabi.make_args(q=q.data_ptr(), k=k.data_ptr(), v=v.data_ptr(), mask=0, out=out.data_ptr(),
                            lse=lse.data_ptr() if return_lse else 0, batch=B, heads=H, heads_k=Hk, seqlen_q=Sq,
                            seqlen_k=Sk, head_dim=d, dtype=_cabi.BF16 if q.dtype == torch.bfloat16 else _cabi.FP16,
-                           device=q.device.index)
+                           device=q.device.index, no_unit_cut=int(bool(single_pass)))
     stream = torch.cuda.current_stream(q.device)
     # the counter the CTAs take their units from and what a split key range needs (any content;
     # private to this call)

@@ -499,5 +499,7 @@ class RecsysOps:
         ``i`` when ``j < valid_lens[b]`` (if given), ``j <= i + Sk - Sq`` (if ``causal``) and
         ``j > i + Sk - Sq - window`` (if ``window > 0``) - the recipes callers build their additive
         masks from (``examples/custom_mask_demo.py:33-65``), evaluated inside the kernel.
-        Bit-identical to ``mha_fwd_with_mask`` on ``masks.rule_mask`` of the same rule."""
+        The result of ``mha_fwd_with_mask`` on ``masks.rule_mask`` of the same rule, up to the rounding of
+        merges: either may split long keys over the GPU, each in its own way.
+        ``masks.rule_attention(..., single_pass=True)`` never does."""
         return self._dispatch(backend, "fa").mha_fwd_rule_mask(q, k, v, bool(causal), int(window), valid_lens)

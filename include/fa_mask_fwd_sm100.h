@@ -56,7 +56,9 @@ enum { FA_SM100_FP16 = 0, FA_SM100_BF16 = 1 };
 enum {
     FA_SM100_NO_TILE_SKIP = 1,  /* visit every key block even where the mask hides it entirely */
     FA_SM100_NO_UNIT_CUT = 2,   /* every (query pair, head, batch) unit is finished by one CTA, so the
-                                 * result does not depend on the number of SMs */
+                                 * result does not depend on the number of SMs (with a mask tensor,
+                                 * together with num_splits = 1; fa_mask_fwd_sm100_rule does not split
+                                 * the keys either then) */
     FA_SM100_NO_HEAD_PAIRS = 4, /* grouped-query heads are neither paired nor, with few query rows, packed
                                  * into shared query tiles: a unit is one head over a 256-row query pair,
                                  * as for ungrouped heads */
@@ -211,7 +213,8 @@ int fa_mask_fwd_sm100_static_scratch(const FaMaskFwdArgs* args, void* stream);
  * that no other call uses until this one has finished; its content does not matter.
  *   fa_mask_fwd_sm100_rule_workspace_bytes(): the call may split long key ranges over the GPU where
  *       too few units would leave SMs idle (fp32 partials, merged; the rounding of the merge is then
- *       the only difference);
+ *       the only difference, and where the cuts lie depends on the number of SMs) - unless args->disable
+ *       has FA_SM100_NO_UNIT_CUT: then this says FA_SM100_RULE_WORKSPACE_BYTES, and it is one pass;
  *   FA_SM100_RULE_WORKSPACE_BYTES: one pass; the counter the CTAs take their units from (units differ
  *       in length under a rule; the call zeroes it on the stream ahead of the kernel);
  *   NULL: one pass, every CTA takes a fixed share of the units (slower where the lengths differ much).

@@ -882,6 +882,27 @@ def test_rule_attention_over_long_keys_is_split(dtype, case):
     assert _cabi.device_status(0, clear=True) == 0
 
 
+@pytest.mark.parametrize("case", [
+    (2, 8, 2, 1, 4100, 128, dict(causal=True)),                   # would be split, two key ranges per CTA
+    (1, 4, 2, 300, 4096, 64, dict(causal=True)),                  # would be cut in pieces
+    (1, 2, 2, 260, 9000, 128, dict(causal=True, window=4000)),
+])
+def test_rule_attention_in_a_single_pass_has_the_bits_of_the_operators(case):
+    """``single_pass`` (FA_SM100_NO_UNIT_CUT below) keeps a rule over long keys whole: the bits of the
+    operator's single pass on the rule mask, whatever the number of SMs."""
+    from custom_ops_b200.masks import rule_attention, rule_mask
+    b, h, hk, sq, sk, d, rule = case
+    q, k, v, _ = make_case(b, h, hk, sq, sk, d, torch.bfloat16, "zero", seed=101)
+    q, k, v = _cuda(q, k, v)
+    want, want_lse, _ = run_cabi(q, k, v, rule_mask(b, sq, sk, **rule), num_splits=1, no_unit_cut=1, want_lse=True)
+    got, got_lse = rule_attention(q, k, v, return_lse=True, single_pass=True, **rule)
+    assert torch.equal(got, want) and torch.equal(got_lse, want_lse)
+    for cut, more in ((0, True), (1, False)):
+        args = _cabi.make_args(batch=b, heads=h, heads_k=hk, seqlen_q=sq, seqlen_k=sk, head_dim=d, dtype=_cabi.BF16,
+                               no_unit_cut=cut)
+        assert (_cabi.rule_workspace_bytes(args, rule.get("window", 0)) > _cabi.RULE_WORKSPACE_BYTES) == more
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("case", [
     # b, h, hk, sq, sk, d: eight heads and more, so that the pre-pass also looks for all-zero blocks
