@@ -85,7 +85,7 @@ class FaMaskFwdPlan(ctypes.Structure):
         ("tile_skip", ctypes.c_int32),
         ("unit_cut", ctypes.c_int32),
         ("head_pairs", ctypes.c_int32),
-        ("reserved0", ctypes.c_int32),
+        ("packed_heads", ctypes.c_int32),
         ("workspace_bytes", ctypes.c_uint64),
     ]
 

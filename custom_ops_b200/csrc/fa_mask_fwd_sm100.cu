@@ -2056,6 +2056,7 @@ static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan, const RuleSpec
     plan->blocks_per_split = bps;
     plan->q_tiles_per_cta = (!one_tile || head_pairs) ? 2 : 1;
     plan->head_pairs = head_pairs ? 1 : 0;
+    plan->packed_heads = ks.pack ? a->heads / ks.H : 0;
     // Units of (split, 256-row query pair, head, batch), or (split, 128-row tile, pair of heads,
     // batch) with head_pairs.  Pair mode is persistent: one CTA per
     // SM takes every grid_x-th unit, so the loads and the first MMA of a unit run under the

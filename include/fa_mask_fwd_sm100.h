@@ -140,14 +140,17 @@ typedef struct FaMaskFwdPlan {
                                  * kernel does not visit them (exact: their weights are 0).  The
                                  * launcher drops the pre-pass for a while after it found nothing to
                                  * skip twice in a row for the same mask buffer and shape. */
-    int32_t unit_cut;           /* P >= 2: there are more single-pass units than CTAs and the R units
-                                 * of the last, partial round are done by P <= SMs / R CTAs each (one
-                                 * piece of the key blocks per CTA, merged through the workspace)
-                                 * instead of leaving most SMs idle; 0: every unit is done by one CTA */
+    int32_t unit_cut;           /* P >= 2: the R single-pass units of the last, partial round - of the
+                                 * only round, where there are fewer units than SMs - are done by
+                                 * P <= SMs / R CTAs each (one piece of the key blocks per CTA, merged
+                                 * through the workspace) instead of leaving most SMs idle; 0: every
+                                 * unit is done by one CTA */
     int32_t head_pairs;         /* 1: grouped-query heads with an even group size: a unit is two heads of
                                  * one KV group over one 128-row query tile (they share every K/V tile
                                  * and every mask tile, and key blocks are skipped per 128 rows) */
-    int32_t reserved0;
+    int32_t packed_heads;       /* n >= 2: with few query rows the rows of n heads of one KV group share
+                                 * query tiles (the whole group, or as many as fill one tile); 0: every
+                                 * head has tiles of its own */
     uint64_t workspace_bytes;
 } FaMaskFwdPlan;
 
@@ -286,7 +289,7 @@ int fa_mask_fwd_sm100_combine_peers(const void* part_table, int64_t part_offset,
 int fa_mask_fwd_sm100_device_status(int32_t device, uint32_t* status, int32_t clear);
 
 /* Number of GPU kernels this library has launched in this process so far (attention, merge,
- * mask re-pitch and tile-skip pre-pass kernels).  For benchmarks that must report how many of
+ * mask re-pitch, tile-skip pre-pass, mask builder and the one that zeroes a rule launch's counter).  For benchmarks that must report how many of
  * the library's kernels ran in a timed region.  No counterpart in the reference. */
 int fa_mask_fwd_sm100_launch_count(uint64_t* launches);
 

@@ -827,7 +827,8 @@ def test_rule_attention_equals_the_operator_on_the_rule_mask(dtype, case):
     (2, 6, 2, 63, 1411, 64, "causal", 1),           # 189 packed rows: two tiles, the second one ragged
     (1, 16, 2, 33, 900, 128, "drop_bias", 1),       # 264 packed rows: a second unit of eight rows
     (1, 8, 2, 1, 4096, 128, "drop10", 5),           # split keys, two splits per CTA, an odd one left over
-    (2, 8, 1, 40, 2053, 64, "random", 3),           # 320 packed rows, split keys
+    (2, 8, 1, 40, 2053, 64, "random", 3),           # split keys: two heads share a tile, four tiles a group
+    (1, 16, 2, 16, 3000, 128, "block", 4),          # ... eight heads fill one exactly
 ])
 def test_packed_heads_equal_separate_heads(dtype, case):
     """With at most 64 query rows the rows of all heads of a KV group share query tiles.  A row's
@@ -835,13 +836,51 @@ def test_packed_heads_equal_separate_heads(dtype, case):
     to the run with one head per unit under the same splits."""
     b, h, hk, sq, sk, d, kind, splits = case
     q, k, v, m = _cuda(*make_case(b, h, hk, sq, sk, d, dtype, kind, seed=61))
-    out, lse, _ = run_cabi(q, k, v, m, want_lse=True, num_splits=splits, no_unit_cut=1)
-    out1, lse1, _ = run_cabi(q, k, v, m, want_lse=True, num_splits=splits, no_unit_cut=1, no_head_pairs=1)
-    if splits == 1 or h // hk * sq <= 128:      # (else one run merges slots in the CTA and the other does not)
-        assert torch.equal(out, out1) and torch.equal(lse, lse1)
+    out, lse, plan = run_cabi(q, k, v, m, want_lse=True, num_splits=splits, no_unit_cut=1)
+    out1, lse1, plan1 = run_cabi(q, k, v, m, want_lse=True, num_splits=splits, no_unit_cut=1, no_head_pairs=1)
+    assert plan.packed_heads >= 2 and plan1.packed_heads == 0
+    assert plan.dual_split == plan1.dual_split == (splits > 1)       # (both merge two splits in the CTA, or neither)
+    assert torch.equal(out, out1) and torch.equal(lse, lse1)
     auto, _, _ = run_cabi(q, k, v, m)
     for o in (out, auto):
         check_against_oracle(o, q, k, v, m, f"packed{case}")
+
+
+@pytest.mark.parametrize("case", [
+    (3, 8, 2, 5, 700, 128, 1), (3, 8, 2, 5, 700, 64, 4),           # one tile: one pass, two splits per CTA
+    (2, 16, 4, 50, 1200, 128, 1), (2, 16, 4, 50, 1200, 128, 0),    # four heads in two tiles; two heads in one, split
+])
+def test_packed_heads_with_one_mask_plane_and_with_fp32_output(case):
+    """Packed heads under a mask whose one plane serves every batch element (batch stride 0), and as the
+    fp32 part with LSE of a split over several GPUs: the bits of the run with a plane per batch element,
+    and that run's output before its rounding."""
+    b, h, hk, sq, sk, d, splits = case
+    q, k, v, m = _cuda(*make_case(b, h, hk, sq, sk, d, torch.bfloat16, "drop10", seed=103))
+    one = m[:1].expand(b, 1, sq, sk)
+    kw = dict(want_lse=True, num_splits=splits, no_unit_cut=1)
+    want, want_lse, plan = run_cabi(q, k, v, one.contiguous(), **kw)
+    assert plan.packed_heads >= 2 and plan.dual_split == (splits != 1)
+    assert one.stride(0) == 0
+    out, lse, _ = run_cabi(q, k, v, one, **kw)
+    assert torch.equal(out, want) and torch.equal(lse, want_lse)
+    part, part_lse, _ = run_cabi(q, k, v, one, out_fp32=True, **kw)
+    assert part.dtype == torch.float32
+    assert torch.equal(part.to(torch.bfloat16), want) and torch.equal(part_lse, want_lse)
+
+
+def test_packed_heads_use_remembered_block_flags():
+    """Packed heads under a mask version: the pre-pass runs once, later calls launch the attention kernel
+    alone and give the same bits."""
+    q, k, v, m = _cuda(*make_case(2, 16, 4, 40, 1411, 128, torch.bfloat16, "zero", seed=107))
+    m = torch.nn.functional.pad(m, (0, 5)).contiguous()                   # rows of 1416: read in place
+    m[..., 256:640] = float("-inf")
+    want, want_lse, plan = run_cabi(q, k, v, m, want_lse=True, num_splits=1, no_unit_cut=1, no_tile_skip=1)
+    assert plan.packed_heads == 4
+    for launches in (2, 1, 1):
+        n0 = _cabi.launch_count()
+        out, lse, plan = run_cabi(q, k, v, m, want_lse=True, num_splits=1, no_unit_cut=1, mask_version=21)
+        assert plan.packed_heads == 4 and plan.tile_skip == 1 and _cabi.launch_count() - n0 == launches
+        assert torch.equal(out, want) and torch.equal(lse, want_lse)
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

@@ -329,6 +329,8 @@ def test_packed_heads_need_no_more_scratch_for_a_given_split(sq, heads_k, num_sp
     for group in (2, 3, 4, 6, 7, 8, 12):
         shape = dict(batch=2, heads=heads_k * group, heads_k=heads_k, seqlen_q=sq, seqlen_k=4096, num_splits=num_splits)
         p, apart = _plan(**shape), _plan(no_head_pairs=1, **shape)
+        fit = max(n for n in range(1, group + 1) if group % n == 0 and (n == 1 or n * sq <= 128))
+        assert p.packed_heads == (fit if fit > 1 else 0) and apart.packed_heads == 0
         assert p.num_splits == apart.num_splits and p.dual_split == apart.dual_split == 1
         assert p.workspace_bytes == apart.workspace_bytes
     assert _plan(batch=2, heads=16, heads_k=2, seqlen_q=64, seqlen_k=4096,
@@ -359,7 +361,7 @@ def test_packed_heads_of_several_tiles_are_split_like_one(heads, heads_k, sq):
             if 8 <= nb < 24 and apart.dual_split:
                 assert p.dual_split == 1 and p.blocks_per_split <= apart.blocks_per_split
             if nb >= 24 or batch == 64:                            # whole groups: several tiles
-                assert p.dual_split == 0 and p.q_tiles_per_cta == 2
+                assert p.dual_split == 0 and p.q_tiles_per_cta == 2 and p.packed_heads == heads // heads_k
 
 
 def test_no_kernel_spills_registers():
