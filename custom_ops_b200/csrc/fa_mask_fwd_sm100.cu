@@ -141,7 +141,11 @@ struct KParams {
     unsigned int wait_kcycles;   // limit of every bounded wait, in units of 1024 SM cycles
     int operands_ready;       // 1: the kernel ahead of this one in the stream is this call's own re-pitch or
                               // pre-pass, which announces its dependents only once every kernel before it
-                              // has finished: q, k and v may be read at once
+                              // has finished: q, k and v may be read at once.  (This rests on completion:
+                              // whoever wrote them has finished, and its writes are in memory, before the
+                              // announcement that lets this kernel start.  The wait, which PTX ties
+                              // visibility to, is executed by the kernel in between, not by these loads;
+                              // they go to the L2.  184.3 us against 187.5, 4 x 1000 x 4099 re-pitched.)
     int mask_bcast;           // 1: one mask plane serves every batch element (batch stride 0)
     int test_stall_mask;      // test only: the mask producer loads nothing, so the waits for the
                               // mask run into their limit and the kernel reports it
@@ -530,7 +534,9 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                 // may still be writing q, k and v, or reading what this launch will overwrite.  Every
                 // role waits for it before its first bounded wait, so that those limits count this
                 // launch's own time only; set-up and the softmax warps' first pass through their code
-                // run under the tail of the kernel before.
+                // run under the tail of the kernel before.  (With operands_ready this producer and the
+                // MMA thread do not wait: their limits also cover this call's own re-pitch or pre-pass,
+                // microseconds of about a second.)
                 if (!p.operands_ready) pdl_wait_prior_grid();
                 Ring ring;                      // next ring slot to fill, over all units
                 int in_flight = 0;              // fills issued (capped), for the drain below
@@ -1034,8 +1040,11 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                     // row's 128 visibility bits are built from the two limits and each score gets
                     // 0 or -inf added (columns beyond Sk lie beyond rule_hi).
                     const int rel_lo = rule_lo - col0, rel_hi = rule_hi - col0;
-                    // (the first pass is voted out inside: a test behind the vote made the kernels spill)
-                    const bool plain = __all_sync(0xffffffffu, rel_lo < 0 && rel_hi >= kBlockN - 1 && !dummy);
+                    // (the first pass takes the other branch; with its test behind the vote the d = 64
+                    // kernels spill, inside it the d = 128 ones take 2 % longer)
+                    bool plain = rel_lo < 0 && rel_hi >= kBlockN - 1;
+                    if constexpr (D == 64) plain = __all_sync(0xffffffffu, plain && !dummy);
+                    else plain = __all_sync(0xffffffffu, plain) && !dummy;
                     if (plain) {
                         scale_only();
                     } else {
@@ -1266,28 +1275,19 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                         const float* part_o = p.cut_part + (static_cast<long long>(slot) * (2 * kBlockM) + tile_row) * D;
                         const float lse_p = ld_cg_f32(p.cut_part + lse_base + static_cast<long long>(slot) * (2 * kBlockM) +
                                                       tile_row);
-                        // out = (a_o * O/l + a_p * o_p) / (a_o + a_p),  a = exp(lse - max lse);
-                        // the merged, normalised row goes back to tensor memory
-                        const float mx = fmaxf(lse_val, lse_p);
-                        float w_o = 0.f, w_p = 0.f;
-                        if (mx != -INFINITY) {
-                            const float a_o = __expf(lse_val - mx), a_p = __expf(lse_p - mx);
-                            const float den = a_o + a_p;
-                            w_o = a_o / den * inv;
-                            w_p = a_p / den;
-                            lse_val = mx + __logf(den);
-                        }
-                        // 64 columns at a time, all of their loads issued before the first is used (one at
-                        // a time they cost a trip to the L2 each).  The four lanes of a quad read line-sized
+                        // All loads of these columns are issued before the first is used (one at a time
+                        // they cost a trip to the L2 each).  The four lanes of a quad read line-sized
                         // pieces of their four rows: the inverse of the stores below, see quad_transpose.
-                        // (The whole row in flight left no registers for what lives across this block: the
-                        // d = 128 kernels for a mask tensor spilled 12 bytes a thread.)
+                        // (With a whole row of d = 128 in flight the kernels for a mask tensor spilled 12
+                        // bytes a thread; with half of one, those under a rule spilled 8.)
+                        constexpr int kAtOnce = RULE ? D / 32 : 2;
                         const int q4 = lane & 3;
+                        float w_o = 0.f, w_p = 0.f;
 #pragma unroll 1
-                        for (int c0 = 0; c0 < D / 32; c0 += 2) {
-                            uint32_t pr[64];
+                        for (int c0 = 0; c0 < D / 32; c0 += kAtOnce) {
+                            uint32_t pr[32 * kAtOnce];
 #pragma unroll
-                            for (int c = 0; c < 2; ++c) {
+                            for (int c = 0; c < kAtOnce; ++c) {
 #pragma unroll
                                 for (int i = 0; i < 4; ++i) {
                                     const float* src = part_o + (i - q4) * D + (c0 + c) * 32 + q4 * 8;
@@ -1298,9 +1298,21 @@ fa_mask_fwd_kernel(const __grid_constant__ CUtensorMap tm_q,
                                     pr[c * 32 + 8 * i + 6] = hi.z; pr[c * 32 + 8 * i + 7] = hi.w;
                                 }
                             }
+                            if (c0 == 0) {
+                                // out = (a_o * O/l + a_p * o_p) / (a_o + a_p),  a = exp(lse - max lse);
+                                // the merged, normalised row goes back to tensor memory
+                                const float mx = fmaxf(lse_val, lse_p);
+                                if (mx != -INFINITY) {
+                                    const float a_o = __expf(lse_val - mx), a_p = __expf(lse_p - mx);
+                                    const float den = a_o + a_p;
+                                    w_o = a_o / den * inv;
+                                    w_p = a_p / den;
+                                    lse_val = mx + __logf(den);
+                                }
+                            }
                             __syncwarp();
 #pragma unroll
-                            for (int c = 0; c < 2; ++c) {
+                            for (int c = 0; c < kAtOnce; ++c) {
                                 uint32_t w[32], oc[32];
 #pragma unroll
                                 for (int i = 0; i < 32; ++i) w[i] = pr[c * 32 + i];
@@ -1977,8 +1989,11 @@ struct RuleSpec {
     bool may_split;                   // the caller brought the workspace that a split or a cut needs
 };
 // Key ranges up to this many blocks run as one pass of whole units under a rule, whose result does
-// not depend on the number of SMs; above it, half-empty launches are split (512 rows, 32 heads in
-// groups of four, 36 blocks: 75.9 -> 52.3 us).
+// not depend on the number of SMs; above it, half-empty launches are split or cut.  The line keeps those
+// results for ordinary lengths; it is not where splitting begins to pay, which is where it does with a mask
+// tensor.  Whole / split from 8 blocks, cut from 12, on (us, d = 128):
+//   one row, 8 x 16 heads in groups of four   8 blocks 17.6 / 18.3   16 30.4 / 18.9   24 42.2 / 20.8   32 - / 22.7
+//   512 rows, 32 heads in groups of four      8 blocks 21.7 / 22.0   16 36.4 / 30.4   24 51.4 / 38.2   36 - / 49.7
 constexpr int kRuleWholeBlocks = 24;
 
 static int make_plan(const FaMaskFwdArgs* a, FaMaskFwdPlan* plan, const RuleSpec* rule = nullptr) {
@@ -2659,6 +2674,7 @@ static int forward(const FaMaskFwdArgs* a, void* workspace, size_t workspace_byt
     unsigned int* ws_unit_counter = reinterpret_cast<unsigned int*>(ws_flags + align256(flag_bytes));
     if (cache == kFlagsHit) {
         // no pre-pass: its other job, resetting the counter the units are handed out from, is done here
+        // (by a memset, so a call that finds its flags is not chained to the kernel before it)
         if (cudaMemsetAsync(ws_unit_counter, 0, sizeof(unsigned int), stream) != cudaSuccess) return cuda_failed(__LINE__);
         kp.block_flags = cached_flags;
         kp.unit_counter = ws_unit_counter;
