@@ -191,6 +191,8 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
 // merging CTA is the one that is dispatched last: whatever it waits for was written by CTAs
 // that are already resident or finished, also when another kernel holds part of the GPU.  (Equal shares of ALL steps, or of the last round's, were
 // measured and lose: the partial traffic of 148 CTAs at once costs more than the idle SMs.)
+enum : int { kPartWhole = 0, kPartTail = 1, kPartHead = 2 };
+
 // Block flags of the pre-pass (0: every key of the block is hidden for all rows of the region), and
 // the mark a visit list carries on the blocks whose mask is zero throughout.
 enum : unsigned char { kFlagMixed = 1, kFlagPlain = 2 };
@@ -200,7 +202,6 @@ constexpr uint32_t kListPlain = 0x8000u;
 // slows the loop even where it never runs (causal, too few heads for marks: 4 heads x 8192 tokens 173.3 us
 // against 161.8, 16 x 4 x 2048 155.4 against 147.7).
 enum : int { kListNone = 0, kListVisit = 1, kListPlainMarks = 2 };
-enum : int { kPartWhole = 0, kPartTail = 1, kPartHead = 2 };
 
 // Unit board: what the scheduler warp publishes about one unit of work, a (split group,
 // 256-row query pair, head, batch) - or (split group, 128-row tile, pair of heads, batch) -
